@@ -4,16 +4,18 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import tempfile
 
 PKG = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libqmcb200.so")
-SOURCES = ["qmcb200.cu", "cusp_fit.c"]
-HEADERS = ["device_common.cuh", "kernels.cuh", "kernels_md.cuh", "kernels_group.cuh", "kernels_rows.cuh", "cusp_fit.h"]
-NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-              "-Xcompiler", "-fPIC", "-shared"]
+SOURCES = ["qmcb200.cu", "move.cu", "group.cu", "md.cu", "full.cu", "rows64.cu", "cusp_fit.c"]
+HEADERS = ["device_common.cuh", "kernels.cuh", "kernels_population.cuh", "population.cuh", "kernels_md.cuh",
+           "kernels_rows.cuh", "group.h", "launches.h", "rows64.h", "cusp_fit.h"]
+ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
+NVCC_FLAGS = [*ARCH_FLAGS, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 
 
 def _nvcc() -> str:
@@ -35,10 +37,19 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not stale():
         return LIB
     os.makedirs(LIBDIR, exist_ok=True)
-    cmd = [_nvcc(), *NVCC_FLAGS, "-o", LIB] + [os.path.join(CSRC, f) for f in SOURCES]
-    if verbose:
-        print(" ".join(cmd), file=sys.stderr)
-    subprocess.check_call(cmd)
+    # the sources side by side: each takes up to two minutes
+    with tempfile.TemporaryDirectory() as tmp:
+        objects = [os.path.join(tmp, f + ".o") for f in SOURCES]
+        jobs = []
+        for f, o in zip(SOURCES, objects):
+            cmd = [_nvcc(), *NVCC_FLAGS, "-c", "-o", o, os.path.join(CSRC, f)]
+            if verbose:
+                print(" ".join(cmd), file=sys.stderr)
+            jobs.append((cmd, subprocess.Popen(cmd)))
+        failed = [(cmd, job.returncode) for cmd, job in jobs if job.wait() != 0]
+        if failed:
+            raise subprocess.CalledProcessError(failed[0][1], failed[0][0])
+        subprocess.check_call([_nvcc(), *ARCH_FLAGS, "-shared", "-o", LIB, *objects])
     return LIB
 
 

@@ -470,7 +470,7 @@ __device__ __forceinline__ int tb_func(const DevSys &S, int A, int i, int j)
 // gradient change on j in pg[(j M + A)][3] (shared scratch, 3 N M doubles);
 // then U_x[j] takes those changes in nucleus order, as a loop over the
 // nuclei of one partner would.
-__device__ __noinline__ void tb_move_lane(const DevSys &S, const double *R, double *Ux, int e, const double *ro,
+static __device__ __noinline__ void tb_move_lane(const DevSys &S, const double *R, double *Ux, int e, const double *ro,
                                           const double *rn, double *acc, double *pg)
 {
   const int N = S.N, M = S.M, lane = threadIdx.x & 31;
@@ -518,7 +518,7 @@ __device__ __noinline__ void tb_move_lane(const DevSys &S, const double *R, doub
 // (QMCThreeBodyJastrow::updateAll, QMcBeaver/src/QMCThreeBodyJastrow.cpp:320-401):
 // lane i sums the gradient on its electron over every partner; U and the
 // laplacian count each pair once (on its higher electron).
-__device__ __noinline__ void tb_full_lane(const DevSys &S, const double *R, double *ux, double *acc)
+static __device__ __noinline__ void tb_full_lane(const DevSys &S, const double *R, double *ux, double *acc)
 {
   const int N = S.N;
   for (int i = threadIdx.x & 31; i < N; i += 32) {

@@ -1,4 +1,4 @@
-// kernels_group.cuh -- the single-electron step of many systems in one launch.
+// group.cu -- the single-electron step of many systems in one launch.
 //
 // Walkers of systems of different sizes (each system a qmcb_handle with its
 // own tables, walker blocks and live list) are processed by one persistent
@@ -12,33 +12,16 @@
 // (one block per member, doing nothing on steps that do not move electron 0),
 // so a batch of steps is a fixed launch sequence that is captured once as a
 // CUDA graph and replayed.
-#pragma once
+#include "group.h"
+#include "kernels_md.cuh"
+#include "kernels_population.cuh"
+#include "launches.h"
 
 namespace qmcb {
-
-constexpr int kGroupMax = 512;  // members of one group
-
-struct GroupMember {
-  DevSys S;
-  Layout L;
-  RunCfg cfg;
-  double *state;
-  int *live, *live_tmp, *free_stack, *ctl;
-  int2 *copies;
-  EnergyCtl *ectl;
-  double *stats;
-  int step0;           // the member's step number at step offset 0
-  int reweight_start;  // reweight_start_step
-  int dmc;
-  int limit_branching;
-  double thr_split, thr_fuse;
-  const double *rows;  // tensor-core rows modes: the step's orbital rows (null: FP64 basis and contraction)
-};
 
 // Member tables of groups that fit (kConst launches): read through the
 // constant cache with warp-uniform indices; groups that do not fit read
 // their table from global memory.
-constexpr int kConstMembers = 84;
 __constant__ GroupMember c_gm[kConstMembers];
 
 __device__ __forceinline__ int group_step(const GroupMember &G, int t) { return G.step0 + t; }
@@ -136,6 +119,31 @@ __global__ void k_energy_group(const GroupMember *__restrict__ gm, int nm, int t
   const GroupMember &G = gm[m];
   if (!G.dmc || group_step(G, t) % G.S.N != 0) return;
   update_energy(G.ectl, G.stats, 1, G.cfg.dyn_dt, G.cfg.dt);
+}
+
+const void *group_move_fn(bool extras, bool ginv, bool cst, bool md)
+{
+  const void *fns[10] = {
+      (const void *)k_move_group<false, false, false, false>, (const void *)k_move_group<true, false, false, false>,
+      (const void *)k_move_group<false, true, false, false>,  (const void *)k_move_group<true, true, false, false>,
+      (const void *)k_move_group<false, false, true, false>,  (const void *)k_move_group<true, false, true, false>,
+      (const void *)k_move_group<false, true, true, false>,   (const void *)k_move_group<true, true, true, false>,
+      (const void *)k_move_group<true, false, false, true>,   (const void *)k_move_group<true, false, true, true>};
+  if (md) return fns[8 + (cst ? 1 : 0)];
+  return fns[(extras ? 1 : 0) + (ginv ? 2 : 0) + (cst ? 4 : 0)];
+}
+
+cudaError_t group_upload_const(const GroupMember *members, int n, int first, cudaStream_t st)
+{
+  return cudaMemcpyToSymbolAsync(c_gm, members, sizeof(GroupMember) * n, sizeof(GroupMember) * first,
+                                 cudaMemcpyHostToDevice, st);
+}
+
+void group_branch(const GroupMember *gm, int nm, int t, cudaStream_t st)
+{
+  k_branch_group<<<nm, 1024, 0, st>>>(gm, t);
+  k_copy_group<<<dim3(64, nm), 256, 0, st>>>(gm, t);
+  k_energy_group<<<(nm + 127) / 128, 128, 0, st>>>(gm, nm, t);
 }
 
 }  // namespace qmcb

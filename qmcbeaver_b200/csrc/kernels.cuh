@@ -11,9 +11,8 @@
 //               inverse update, ratio sums, incremental Jastrow and
 //               potential, psi quantities, Metropolis test, DMC reweight and
 //               observables, commit on accept
-//   k_branch    nonunit-weight branching of the live list (single CTA)
-//   k_copy      state copies for split walkers
-//   k_energy    E_est / E_T update after a branching step
+// The population's kernels (branching, copies, energies, read back) are in
+// kernels_population.cuh.
 #pragma once
 
 #include "device_common.cuh"
@@ -733,26 +732,9 @@ __device__ inline double umrigar_log_gf(const UmrigarFrame &F, const RunCfg &cfg
   return m + log(exp(lg - m) + exp(ls - m));
 }
 
-// Proposal of electron e and ln G(R -> R') over all electrons (the
-// unmoved ones contribute their stay-in-place density; cfg.exact_gf: the
-// moved electron only).
-__device__ __noinline__ void umrigar_propose(const DevSys &S, const RunCfg &cfg, int slot, int step, int e, int N,
-                                             const double *R, const double *mgo, double *rn, double *log_fwd,
-                                             double *u_acc)
+// The frame's proposal from the uniforms u[0..5].
+__device__ __forceinline__ void umrigar_draw(const UmrigarFrame &F, const RunCfg &cfg, const double *u, double *rn)
 {
-  const int lane = threadIdx.x & 31;
-  // lanes 0-3 draw two uniforms each from their own Philox counters
-  double u[8];
-  {
-    const U4 c = philox4x32(U4{(uint32_t)slot, (uint32_t)step, (uint32_t)(8 + (lane & 3)), 0x0A7E5A21u}, cfg.seed);
-    const double ua = u01(c.x, c.y), ub = u01(c.z, c.w);
-    for (int k = 0; k < 4; k++) {
-      u[2 * k] = __shfl_sync(QMCB_FULL_MASK, ua, k);
-      u[2 * k + 1] = __shfl_sync(QMCB_FULL_MASK, ub, k);
-    }
-  }
-  UmrigarFrame F;
-  umrigar_frame(S, cfg, R + 3 * e, mgo + 3 * e, F);
   if (u[0] < F.pg) {
     // Gaussian around the drifted centre (Box-Muller from u[1..4])
     const double r1 = sqrt(-2.0 * log(u[1])), r2 = sqrt(-2.0 * log(u[3]));
@@ -769,6 +751,29 @@ __device__ __noinline__ void umrigar_propose(const DevSys &S, const RunCfg &cfg,
     rn[1] = F.A[1] + r * sin(theta) * sin(phi);
     rn[2] = F.A[2] + r * cos(theta);
   }
+}
+
+// Proposal of electron e and ln G(R -> R') over all electrons (the
+// unmoved ones contribute their stay-in-place density; cfg.exact_gf: the
+// moved electron only).
+static __device__ __noinline__ void umrigar_propose(const DevSys &S, const RunCfg &cfg, int slot, int step, int e, int N,
+                                             const double *R, const double *mgo, double *rn, double *log_fwd,
+                                             double *u_acc)
+{
+  const int lane = threadIdx.x & 31;
+  // lanes 0-3 draw two uniforms each from their own Philox counters
+  double u[8];
+  {
+    const U4 c = philox4x32(U4{(uint32_t)slot, (uint32_t)step, (uint32_t)(8 + (lane & 3)), 0x0A7E5A21u}, cfg.seed);
+    const double ua = u01(c.x, c.y), ub = u01(c.z, c.w);
+    for (int k = 0; k < 4; k++) {
+      u[2 * k] = __shfl_sync(QMCB_FULL_MASK, ua, k);
+      u[2 * k + 1] = __shfl_sync(QMCB_FULL_MASK, ub, k);
+    }
+  }
+  UmrigarFrame F;
+  umrigar_frame(S, cfg, R + 3 * e, mgo + 3 * e, F);
+  umrigar_draw(F, cfg, u, rn);
   *u_acc = u[6];
   double part = 0.0;
   for (int i = lane; i < N; i += 32) {
@@ -785,7 +790,7 @@ __device__ __noinline__ void umrigar_propose(const DevSys &S, const RunCfg &cfg,
 
 // ln G(R' -> R): frames of the new positions R' with the new drift, density
 // at the old positions (the moved electron's old position is ro).
-__device__ __noinline__ double umrigar_log_reverse(const DevSys &S, const RunCfg &cfg, int e, int N, const double *Rn,
+static __device__ __noinline__ double umrigar_log_reverse(const DevSys &S, const RunCfg &cfg, int e, int N, const double *Rn,
                                                    const double *mg, const double *ro)
 {
   double part = 0.0;
@@ -796,6 +801,19 @@ __device__ __noinline__ double umrigar_log_reverse(const DevSys &S, const RunCfg
     part += umrigar_log_gf(F, cfg, i == e ? ro : Rn + 3 * i);
   }
   return warp_sum(part);
+}
+
+// A Gaussian sample by Box-Muller in single precision: the proposal only
+// needs a Gaussian sample, not a particular one (the random streams differ
+// from the reference's ran1 in any case).
+__device__ __forceinline__ float gaussian_draw(const U4 &c)
+{
+  const float u1 = ((float)(c.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
+  const float u2 = (float)(c.y >> 8) * (1.0f / 16777216.0f);
+  const float rad = sqrtf(-2.0f * __logf(u1));
+  float sn, cs;
+  __sincosf(6.2831853f * u2, &sn, &cs);
+  return rad * cs;
 }
 
 // New position of electron e: the walker's own Philox stream and the drift
@@ -822,15 +840,7 @@ __device__ __forceinline__ void propose_move(const DevSys &S, const RunCfg &cfg,
     double zr, z[3];
     {
       const U4 c = philox4x32(U4{(uint32_t)slot, (uint32_t)step, (uint32_t)(lane & 3), 0x51ED2701u}, cfg.seed);
-      // Box-Muller in single precision: the proposal only needs a Gaussian
-      // sample, not a particular one (the random streams differ from the
-      // reference's ran1 in any case)
-      const float u1 = ((float)(c.x >> 8) + 0.5f) * (1.0f / 16777216.0f);
-      const float u2 = (float)(c.y >> 8) * (1.0f / 16777216.0f);
-      const float rad = sqrtf(-2.0f * __logf(u1));
-      float sn, cs;
-      __sincosf(6.2831853f * u2, &sn, &cs);
-      zr = (lane & 3) == 3 ? u01(c.z, c.w) : (double)(rad * cs);
+      zr = (lane & 3) == 3 ? u01(c.z, c.w) : (double)gaussian_draw(c);
     }
     z[0] = __shfl_sync(QMCB_FULL_MASK, zr, 0);
     z[1] = __shfl_sync(QMCB_FULL_MASK, zr, 1);
@@ -1524,307 +1534,6 @@ __global__ void __launch_bounds__(128, kGInv ? 3 : 5) k_move(DevSys S, Layout L,
   if (wi >= nw) return;
   move_walker<kMetropolis, TS, TI, kExtras, kGInv>(S, L, cfg, state, slots, wi, smem + (size_t)warp * L.mv_stride,
                                                    R_in, mv, ectl, stats, out);
-}
-
-// ------------------------------------------------------------------------
-// Nonunit-weight branching (QMCRun::nonunitWeightBranching,
-// QMcBeaver/src/QMCRun.cpp:740-814) on the live slot list, one CTA of
-// 1024 threads.  Walkers above the branching threshold split in two with
-// half the weight each (the copy is appended to the list), walkers below
-// 0.01 die, walkers below the fusion threshold are paired in list order and
-// one of each pair survives with the sum of the weights (probability
-// w1 / (w1 + w2) for the first; the uniform draw of a pair is keyed by
-// (seed, position of its first member in the live list, step)).  The split
-// test uses the weight before fusion, so a fused survivor does not split in
-// the same pass.  Dead slots go on the free stack; copies
-// take slots from it and are written to the copy list for k_copy.
-// ctl: [0] n_live, [1] n_free, [2] n_copies.
-// QMCWalker::branchRecommended (limit_branching): no split for a walker that
-// has not moved for more than 4 steps, whose weight grows too fast
-// (dW^(age+1) > 5), that is heavy (> 100) and still growing (> 1.5), or whose
-// local energy is more than 100x off the input energy.
-__device__ __forceinline__ bool branch_recommended(const double *sc, double e_orig, int limit)
-{
-  if (!limit) return true;
-  const double age = sc[SC_AGE], W = sc[SC_WEIGHT], dW = sc[SC_DW];
-  const double growth = pow(dW, age + 1.0);
-  bool ok = true;
-  if (age > 4.0) ok = false;
-  if (growth > 5.0)
-    ok = false;
-  else if (W > 100.0 && growth > 1.5)
-    ok = false;
-  if (fabs((sc[SC_EL] - e_orig) / e_orig) > 100.0) ok = false;
-  return ok;
-}
-
-__device__ __forceinline__ void branch_block(double *state, const Layout &L, int *live, int *live_tmp,
-                                             int *free_stack, int *ctl, int2 *copies, double thr_split,
-                                             double thr_fuse, uint64_t seed, int step, double *stats, double e_orig,
-                                             int limit_branching)
-{
-  __shared__ int s_warp[32];
-  __shared__ int s_base[4];
-  __shared__ double s_wsum[32];
-  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-  const int n = ctl[0];
-  int nfree = ctl[1];
-  // pass 1: pair fusion candidates in list order and decide
-  int cand_base = 0;
-  for (int c0 = 0; c0 < n; c0 += 1024) {
-    int i = c0 + tid;
-    int slot = i < n ? live[i] : -1;
-    double w = slot >= 0 ? state[(size_t)slot * L.stride + L.sc + SC_WEIGHT] : 0.0;
-    int is_c = (slot >= 0 && w <= thr_split && w >= 0.01 && w < thr_fuse) ? 1 : 0;
-    // block exclusive scan of is_c
-    unsigned b = __ballot_sync(QMCB_FULL_MASK, is_c);
-    int wpre = __popc(b & ((1u << lane) - 1));
-    if (lane == 31) s_warp[wid] = wpre + is_c;
-    __syncthreads();
-    if (wid == 0) {
-      int v = s_warp[lane], x = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(QMCB_FULL_MASK, x, o);
-        if (lane >= o) x += y;
-      }
-      s_warp[lane] = x - v;
-      if (lane == 31) s_base[0] = x;
-    }
-    __syncthreads();
-    int rank = cand_base + s_warp[wid] + wpre;  // global candidate rank
-    int total = s_base[0];
-    // candidate ranks are global over the whole list, so pairs (0,1), (2,3)
-    // ... may straddle chunk boundaries.
-    if (is_c) live_tmp[rank] = i;
-    __syncthreads();
-    cand_base += total;
-  }
-  __syncthreads();
-  // decide pairs: candidate 2m and 2m+1
-  for (int m = tid; 2 * m + 1 < cand_base; m += 1024) {
-    int ia = live_tmp[2 * m], ib = live_tmp[2 * m + 1];
-    int sa = live[ia], sb = live[ib];
-    double *wa = &state[(size_t)sa * L.stride + L.sc + SC_WEIGHT];
-    double *wb = &state[(size_t)sb * L.stride + L.sc + SC_WEIGHT];
-    double w1 = *wa, w2 = *wb, w3 = w1 + w2;
-    double u[4];
-    rng_uniform4(seed, (uint32_t)ia, (uint32_t)step, 7u, u);
-    if (u[0] < w1 / w3) {
-      *wa = w3;
-      *wb = -1.0;  // marked dead
-      wa[SC_FUSED - SC_WEIGHT] = 1.0;
-    } else {
-      *wb = w3;
-      *wa = -1.0;
-      wb[SC_FUSED - SC_WEIGHT] = 1.0;
-    }
-  }
-  __syncthreads();
-  // pass 2: survivors keep list order; dead slots to the free stack; splits append copies
-  int out_base = 0, split_base = 0;
-  // first count survivors + kills to know where split copies go and how many slots free
-  for (int c0 = 0; c0 < n; c0 += 1024) {
-    int i = c0 + tid;
-    int slot = i < n ? live[i] : -1;
-    double w = slot >= 0 ? state[(size_t)slot * L.stride + L.sc + SC_WEIGHT] : 0.0;
-    int dead = (slot >= 0 && w < 0.01) ? 1 : 0;
-    int keep = (slot >= 0 && !dead) ? 1 : 0;
-    unsigned bk = __ballot_sync(QMCB_FULL_MASK, keep), bd = __ballot_sync(QMCB_FULL_MASK, dead);
-    int pk = __popc(bk & ((1u << lane) - 1)), pd = __popc(bd & ((1u << lane) - 1));
-    if (lane == 31) s_warp[wid] = ((pk + keep) << 16) | (pd + dead);
-    __syncthreads();
-    if (wid == 0) {
-      int v = s_warp[lane];
-      int vk = v >> 16, vd = v & 0xffff, xk = vk, xd = vd;
-      for (int o = 1; o < 32; o <<= 1) {
-        int yk = __shfl_up_sync(QMCB_FULL_MASK, xk, o), yd = __shfl_up_sync(QMCB_FULL_MASK, xd, o);
-        if (lane >= o) {
-          xk += yk;
-          xd += yd;
-        }
-      }
-      s_warp[lane] = ((xk - vk) << 16) | (xd - vd);
-      if (lane == 31) {
-        s_base[1] = xk;
-        s_base[2] = xd;
-      }
-    }
-    __syncthreads();
-    int ok = s_warp[wid] >> 16, od = s_warp[wid] & 0xffff;
-    if (keep) live_tmp[out_base + ok + pk] = slot;
-    if (dead) free_stack[nfree + od + pd] = slot;
-    int tk = s_base[1], td = s_base[2];
-    __syncthreads();
-    out_base += tk;
-    nfree += td;
-  }
-  __syncthreads();
-  // splits among survivors (in new list order), appended at the end
-  int n_keep = out_base;
-  double wsum_part = 0.0;
-  for (int c0 = 0; c0 < n_keep; c0 += 1024) {
-    int i = c0 + tid;
-    int slot = i < n_keep ? live_tmp[i] : -1;
-    double *wp = slot >= 0 ? &state[(size_t)slot * L.stride + L.sc + SC_WEIGHT] : nullptr;
-    double w = wp ? *wp : 0.0;
-    // the split test reads the weight before fusion, as the reference's single
-    // pass does: the survivor of a fused pair (weight below the fusion
-    // threshold before) never splits in the same pass
-    const bool fused = wp && wp[SC_FUSED - SC_WEIGHT] != 0.0;
-    if (fused) wp[SC_FUSED - SC_WEIGHT] = 0.0;
-    int sp = (slot >= 0 && !fused && w > thr_split &&
-              branch_recommended(state + (size_t)slot * L.stride + L.sc, e_orig, limit_branching)) ? 1 : 0;
-    unsigned bs = __ballot_sync(QMCB_FULL_MASK, sp);
-    int ps = __popc(bs & ((1u << lane) - 1));
-    if (lane == 31) s_warp[wid] = ps + sp;
-    __syncthreads();
-    if (wid == 0) {
-      int v = s_warp[lane], x = v;
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(QMCB_FULL_MASK, x, o);
-        if (lane >= o) x += y;
-      }
-      s_warp[lane] = x - v;
-      if (lane == 31) s_base[3] = x;
-    }
-    __syncthreads();
-    int r = split_base + s_warp[wid] + ps;
-    if (sp) {
-      if (r < nfree) {
-        int dst = free_stack[nfree - 1 - r];
-        *wp = w * 0.5;
-        copies[r] = make_int2(slot, dst);
-        live_tmp[n_keep + r] = dst;
-        wsum_part += w;  // both halves
-      } else {
-        wsum_part += w;  // no free slot: keep the walker whole
-      }
-    } else if (slot >= 0) {
-      wsum_part += w;
-    }
-    int ts = s_base[3];
-    __syncthreads();
-    split_base += ts;
-  }
-  int n_split = min(split_base, nfree);
-  __syncthreads();
-  for (int i = tid; i < n_keep + n_split; i += 1024) live[i] = live_tmp[i];
-  double ws = warp_sum(wsum_part);
-  if (lane == 0) s_wsum[wid] = ws;
-  __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-    for (int k = 0; k < 32; k++) t += s_wsum[k];
-    stats[ST_FINAL_W] = t;
-    ctl[0] = n_keep + n_split;
-    ctl[1] = nfree - n_split;
-    ctl[2] = n_split;
-  }
-}
-
-__global__ void __launch_bounds__(1024) k_branch(double *state, Layout L, int *live, int *live_tmp, int *free_stack,
-                                                 int *ctl, int2 *copies, double thr_split, double thr_fuse,
-                                                 uint64_t seed, int step, double *stats, double e_orig,
-                                                 int limit_branching)
-{
-  branch_block(state, L, live, live_tmp, free_stack, ctl, copies, thr_split, thr_fuse, seed, step, stats, e_orig,
-               limit_branching);
-}
-
-// Copies whole walker blocks for the splits recorded by k_branch; the copy
-// keeps the halved weight already written to the source.
-__device__ __forceinline__ void copy_blocks(double *state, const Layout &L, const int2 *copies, const int *ctl,
-                                            int first, int stride)
-{
-  const int nc = ctl[2];
-  for (int c = first; c < nc; c += stride) {
-    int2 p = copies[c];
-    const double *src = state + (size_t)p.x * L.stride;
-    double *dst = state + (size_t)p.y * L.stride;
-    for (int t = threadIdx.x; t < L.stride; t += blockDim.x) dst[t] = src[t];
-  }
-}
-
-__global__ void k_copy(double *state, Layout L, const int2 *copies, const int *ctl)
-{
-  copy_blocks(state, L, copies, ctl, blockIdx.x, gridDim.x);
-}
-
-// E_est from the running weighted energy average and
-// E_T = E_est - c ln(W / W0) (QMCManager::updateEstimatedEnergy /
-// updateTrialEnergy, QMcBeaver/src/QMCManager.cpp:2247-2310).
-// dyn_dt: also the effective time step dt <w p dR^2> / <w dR^2>
-// (QMCDerivativeProperties::getEffectiveTimeStep, QMcBeaver/src/QMCDerivativeProperties.cpp:25-42).
-__device__ __forceinline__ void update_energy(EnergyCtl *ectl, const double *stats, int min_samples_ok, int dyn_dt,
-                                              double dt)
-{
-  if (dyn_dt && stats[ST_RUN_SUM_WD2] > 1e-20) ectl->dt_eff = dt * stats[ST_RUN_SUM_WPD2] / stats[ST_RUN_SUM_WD2];
-  double sw = stats[ST_RUN_SUM_W];
-  // E_est follows the running average once it holds 100 samples
-  // (QMCManager::updateEstimatedEnergy, QMcBeaver/src/QMCManager.cpp:2247-2261)
-  if (min_samples_ok && sw > 0.0 && stats[ST_RUN_COUNT] >= 100.0) ectl->e_est = stats[ST_RUN_SUM_WE] / sw;
-  double ratio = stats[ST_FINAL_W] / ectl->target_weight;
-  double lr = ratio > 1e-250 ? log(ratio) : 0.0;
-  ectl->e_trial = ectl->e_est - ectl->pop_control * lr;
-}
-
-__global__ void k_energy(EnergyCtl *ectl, const double *stats, int min_samples_ok, int dyn_dt, double dt)
-{
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  update_energy(ectl, stats, min_samples_ok, dyn_dt, dt);
-}
-
-// Packs R, weight, E_L, log|psi|, sign of the first n live walkers into
-// out[n][3N + 4] for one device-to-host copy.
-__global__ void k_gather(const double *state, Layout L, int N, const int *live, int n, double *out)
-{
-  const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = lane_id();
-  if (w >= n) return;
-  const double *blk = state + (size_t)live[w] * L.stride;
-  double *o = out + (size_t)w * (3 * N + 4);
-  for (int t = lane; t < 3 * N; t += 32) o[t] = blk[L.R + t];
-  if (lane == 0) {
-    const double *sc = blk + L.sc;
-    o[3 * N] = sc[SC_WEIGHT];
-    o[3 * N + 1] = sc[SC_EL];
-    o[3 * N + 2] = sc[SC_LOGDET_A] + sc[SC_LOGDET_B] + sc[SC_U];
-    o[3 * N + 3] = sc[SC_SIGN_A] * sc[SC_SIGN_B];
-  }
-}
-
-// Sets the weights of the first n live walkers.
-__global__ void k_set_weights(double *state, Layout L, const int *live, int n, const double *w)
-{
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    state[(size_t)live[i] * L.stride + L.sc + SC_WEIGHT] = w[i];
-}
-
-// Per-walker evaluate outputs moved from the device buffer into mapped
-// page-locked host arrays with consecutive threads on consecutive elements,
-// so the stores cross the bus as full packets (the evaluate kernels store a
-// walker's scalars from one lane, one 8-byte packet each).  Segment
-// blockIdx.y: bytes[y] bytes from src[y] to dst[y]; whole 8-byte words when
-// both ends and the length allow it, bytes otherwise.
-struct PutList {
-  const void *src[8];
-  void *dst[8];
-  size_t bytes[8];
-};
-
-__global__ void k_put_outputs(PutList P)
-{
-  const int y = blockIdx.y;
-  const size_t n = P.bytes[y];
-  const size_t i0 = (size_t)blockIdx.x * blockDim.x + threadIdx.x, di = (size_t)gridDim.x * blockDim.x;
-  if (((uintptr_t)P.src[y] | (uintptr_t)P.dst[y] | n) % 8 == 0) {
-    const unsigned long long *s = (const unsigned long long *)P.src[y];
-    unsigned long long *d = (unsigned long long *)P.dst[y];
-    for (size_t i = i0; i < n / 8; i += di) d[i] = s[i];
-  } else {
-    const unsigned char *s = (const unsigned char *)P.src[y];
-    unsigned char *d = (unsigned char *)P.dst[y];
-    for (size_t i = i0; i < n; i += di) d[i] = s[i];
-  }
 }
 
 }  // namespace qmcb

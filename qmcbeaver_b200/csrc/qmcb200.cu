@@ -3,11 +3,12 @@
 // Host side of include/qmcb200.h: device tables for the molecular system,
 // the per-walker state blocks, the live-walker list used by DMC branching,
 // and the launch sequence of one Monte Carlo step.  Kernels are in
-// kernels.cuh.  No CPU fallback: every entry point fails with QMCB_E_CUDA
+// kernels.cuh and the files that launches.h names.  No CPU fallback: every entry point fails with QMCB_E_CUDA
 // when no CUDA device is usable.
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -19,18 +20,15 @@
 
 #include "../../include/qmcb200.h"
 #include "cusp_fit.h"
+#include "group.h"
 #include "kernels.cuh"
 #include "kernels_md.cuh"
-#include "kernels_group.cuh"
 #include "kernels_rows.cuh"
+#include "launches.h"
+#include "population.cuh"
+#include "rows64.h"
 
 using namespace qmcb;
-
-// Mixed precision: FP32 basis values, orbital rows and contraction; the
-// inverse and its Sherman-Morrison update in MIXED_TI.
-#ifndef MIXED_TI
-#define MIXED_TI double
-#endif
 
 namespace {
 
@@ -68,6 +66,12 @@ struct qmcb_handle {
   int bf_ksteps = 0;
   int rows_n = 0, rows_num = 0;  // the last tensor-core rows launch: orbitals per row, list capacity
   size_t smem_rows = 0, smem_prep = 0;
+  // batched FP64 rows (kernels_rows64.cuh): tables, rows buffer [walker][5][n]
+  Rows64 r64{};
+  int rows64_from = INT_MAX;  // FP64 single-electron moves of this many walkers take their rows from k_rows64
+  int4 *d_r64_chunk = nullptr;
+  double *d_r64_rec = nullptr;
+  double *d_r64_ct[2] = {nullptr, nullptr}, *d_rows64 = nullptr;
   Layout lay_rows{};  // move-kernel scratch without the basis rows
   double *d_pade = nullptr;
   int2 *d_pade_len = nullptr;
@@ -396,19 +400,140 @@ void *g_noalloc_i_addr[64];
 
 // One launch of the single-determinant move kernel in the walker state's
 // precision, with the cusp / three-body code only when the system has them.
-template <bool kMetropolis, typename TS, typename TI, bool kExtras>
-static void launch_move_g(qmcb_handle *h, const dim3 &g, const dim3 &b, size_t sm, cudaStream_t st, const RunCfg &cfg,
-                          const int *slots, int num, const int *d_num, const double *R_in, const MoveArgs &mv,
-                          const EvalOut &o)
+static void launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extras, const dim3 &g, const dim3 &b,
+                          size_t sm, cudaStream_t st, const RunCfg &cfg, const int *slots, int num, const int *d_num,
+                          const double *R_in, const MoveArgs &mv, const EvalOut &o)
 {
-  // with rows from the tensor cores the scratch has no basis rows
+  // with rows from a batched kernel the scratch has no basis rows
   const Layout &L = mv.rows ? h->lay_rows : h->lay;
-  if (h->ginv)
-    k_move<kMetropolis, TS, TI, kExtras, true><<<g, b, sm, st>>>(h->sys, L, cfg, h->d_state, slots, num, d_num,
-                                                                 R_in, mv, h->d_ectl, h->d_stats, o);
-  else
-    k_move<kMetropolis, TS, TI, kExtras, false><<<g, b, sm, st>>>(h->sys, L, cfg, h->d_state, slots, num, d_num,
-                                                                  R_in, mv, h->d_ectl, h->d_stats, o);
+  launch_kernel(move_fn(metropolis, mixed, extras, h->ginv), g, b, sm, st, h->sys, L, cfg, h->d_state, slots, num,
+                d_num, R_in, mv, h->d_ectl, h->d_stats, o);
+}
+
+// The chunks of k_rows64 (struct Rows64): shells dealt, largest first, to the
+// emptiest chunk with room (so that every chunk holds a like mix of cheap and
+// dear shells), sorted by cost within a chunk.  Complete s, p and d shells of
+// at most three primitives take the kernel's fast kinds; any other shell of
+// more than kR64Chunk functions is cut.  r64.nchunk
+// stays 0 (the kernel is not used) when a shell's record would not fit.
+static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells, const std::vector<int2> &fn,
+                                 const std::vector<double4> &nuc, const std::vector<double> &pexp,
+                                 const std::vector<double> &pcoef, const std::vector<double> ct[2], const int nact[2])
+{
+  struct Item {
+    int atom, kind, L, np, off;
+    std::vector<int> members;  // functions in the record's order
+  };
+  const auto same = [&](int k, int l, int np) {
+    return std::memcmp(&pcoef[fn[k].y], &pcoef[fn[l].y], sizeof(double) * np) == 0;
+  };
+  const auto doubles = [](const Item &it) {
+    const int nmem = (int)it.members.size();
+    return it.kind == kR64Any ? 5 + it.np + nmem * (it.np + 1) : 7 + 3 * nmem;
+  };
+  std::vector<Item> items;
+  for (const int4 &sh : shells) {
+    const int nmem = sh.z & 0xff, L = (sh.z >> 8) & 0xff, np = sh.z >> 16;
+    Item it{sh.x, kR64Any, L, np, sh.w, {}};
+    // the functions of a complete shell in the order of its kind
+    const int order[3][6] = {{0}, {1, 1 << 8, 1 << 16}, {2, 2 << 8, 2 << 16, 1 | 1 << 8, 1 | 1 << 16, 1 << 8 | 1 << 16}};
+    if (L <= 2 && np <= 3 && nmem == (L + 1) * (L + 2) / 2) {
+      for (int m = 0; m < nmem; m++)
+        for (int k = sh.y; k < sh.y + nmem; k++)
+          if (fn[k].x == order[L][m]) it.members.push_back(k);
+      if ((int)it.members.size() == nmem) {
+        it.kind = L;
+        items.push_back(it);
+        continue;
+      }
+    }
+    for (int m = 0; m < nmem; m += kR64Chunk) {
+      it.members.clear();
+      for (int k = m; k < std::min(nmem, m + kR64Chunk); k++) it.members.push_back(sh.y + k);
+      items.push_back(it);
+    }
+  }
+  for (const Item &it : items)
+    if (doubles(it) >= kR64RecMax) return cudaSuccess;
+  std::stable_sort(items.begin(), items.end(),
+                   [](const Item &a, const Item &b) { return a.members.size() > b.members.size(); });
+  std::vector<std::vector<Item>> chunks((h->K + kR64Chunk - 1) / kR64Chunk);
+  std::vector<int> fill(chunks.size(), 0), size(chunks.size(), 0);
+  for (const Item &it : items) {
+    const int nmem = (int)it.members.size();
+    int best = -1;
+    for (size_t c = 0; c < chunks.size(); c++)
+      if (fill[c] + nmem <= kR64Chunk && size[c] + doubles(it) < kR64RecMax && (best < 0 || fill[c] < fill[best]))
+        best = (int)c;
+    if (best < 0) {
+      best = (int)chunks.size();
+      chunks.emplace_back();
+      fill.push_back(0);
+      size.push_back(0);
+    }
+    chunks[best].push_back(it);
+    fill[best] += nmem;
+    size[best] += doubles(it);
+  }
+  const auto words = [](int hi, int lo) {
+    const uint64_t v = ((uint64_t)(uint32_t)hi << 32) | (uint32_t)lo;
+    double d;
+    std::memcpy(&d, &v, sizeof(d));
+    return d;
+  };
+  std::vector<int4> chunk;
+  std::vector<double> rec, pct[2];
+  int row = 0;
+  for (size_t c = 0; c < chunks.size(); c++) {
+    auto &items_c = chunks[c];
+    // an exponential costs about eight members' own work
+    std::stable_sort(items_c.begin(), items_c.end(), [](const Item &a, const Item &b) {
+      return (int)a.members.size() + 8 * a.np > (int)b.members.size() + 8 * b.np;
+    });
+    const int padded = (fill[c] + 7) & ~7, start = (int)rec.size();
+    chunk.push_back(make_int4((int)items_c.size(), start, fill[c] | (padded << 16), row));
+    for (int sp = 0; sp < 2; sp++) pct[sp].resize((size_t)(row + padded) * rows64_ldb(nact[sp]), 0.0);
+    rec.resize(rec.size() + items_c.size());
+    int col = 0;
+    for (size_t i = 0; i < items_c.size(); i++) {
+      const Item &it = items_c[i];
+      const int nmem = (int)it.members.size();
+      rec[start + i] = words((int)rec.size() - start, col | (nmem << 8) | (it.kind << 16));
+      rec.insert(rec.end(), {nuc[it.atom].x, nuc[it.atom].y, nuc[it.atom].z});
+      if (it.kind == kR64Any) rec.push_back(words(it.np, it.L));
+      const int pad = it.kind == kR64Any ? 0 : 3 - it.np;
+      rec.insert(rec.end(), pexp.begin() + it.off, pexp.begin() + it.off + it.np);
+      rec.insert(rec.end(), pad, 0.0);
+      for (int m = 0; m < nmem; m++, col++) {
+        const int k = it.members[m], f = fn[k].y;
+        if (it.kind == kR64Any) {
+          const bool repeat = m > 0 && same(k, it.members[m - 1], it.np);
+          rec.push_back(words(0, fn[k].x | (repeat ? 1 << 24 : 0)));
+        }
+        rec.insert(rec.end(), pcoef.begin() + f, pcoef.begin() + f + it.np);
+        rec.insert(rec.end(), pad, 0.0);
+        for (int sp = 0; sp < 2; sp++)
+          for (int o = 0; o < nact[sp]; o++)
+            pct[sp][(size_t)(row + col) * rows64_ldb(nact[sp]) + o] = ct[sp][(size_t)k * nact[sp] + o];
+      }
+    }
+    if (rec.size() & 1) rec.push_back(0.0);
+    h->r64.rec_max = std::max(h->r64.rec_max, (int)rec.size() - start);
+    row += padded;
+  }
+  chunk.push_back(make_int4(0, (int)rec.size(), 0, row));
+  cudaError_t e = upload(&h->d_r64_chunk, chunk);
+  if (e == cudaSuccess) e = upload(&h->d_r64_rec, rec);
+  for (int sp = 0; sp < 2; sp++)
+    if (e == cudaSuccess) e = upload(&h->d_r64_ct[sp], pct[sp]);
+  h->r64.nchunk = (int)chunks.size();
+  h->r64.chunk = h->d_r64_chunk;
+  h->r64.rec = h->d_r64_rec;
+  for (int sp = 0; sp < 2; sp++) {
+    h->r64.ct[sp] = h->d_r64_ct[sp];
+    h->r64.ldb[sp] = rows64_ldb(nact[sp]);
+  }
+  return e;
 }
 
 // Walker state written under QMCB_PREC_FP64 serves the tensor-core rows modes too.
@@ -418,6 +543,18 @@ static int state_kind(int prec) { return prec == QMCB_PREC_MIXED ? QMCB_PREC_MIX
 static bool rows_mode(int prec)
 {
   return prec == QMCB_PREC_INT8_SLICES || prec == QMCB_PREC_BF16_TC || prec == QMCB_PREC_BF16X3_TC;
+}
+
+// Whether FP64 moves of `cap` list entries take their rows from k_rows64.
+static bool rows64_moves(const qmcb_handle *h, int cap)
+{
+  return h->params.precision == QMCB_PREC_FP64 && cap >= h->rows64_from;
+}
+
+// Whether the steps of all a handle's walkers take rows from a batched kernel.
+static bool batched_rows(const qmcb_handle *h)
+{
+  return rows_mode(h->params.precision) || rows64_moves(h, h->max_walkers);
 }
 
 // The batched orbital rows of one single-electron step (the tensor-core
@@ -495,40 +632,30 @@ static void launch_move(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
     mv.rows = h->d_rows_out;
     const dim3 g((cap + h->wpb_rows - 1) / h->wpb_rows), b(32 * h->wpb_rows);
     ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-    if (extras)
-      launch_move_g<kMetropolis, double, double, true>(h, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
-    else
-      launch_move_g<kMetropolis, double, double, false>(h, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
+    launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
+    ps.end(st);
+    return;
+  }
+  if (rows64_moves(h, cap)) {
+    {
+      ProfScope ps(h, QMCB_KERNEL_ROWS_PREP, st);
+      rows64_launch(kMetropolis ? R64_PROPOSE : R64_GIVEN, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num,
+                    d_num, R_in, mv, mv.e < h->sys.na ? 0 : 1, h->d_rows64);
+      ps.end(st);
+    }
+    mv.rows = h->d_rows64;
+    const dim3 g((cap + h->wpb_rows - 1) / h->wpb_rows), b(32 * h->wpb_rows);
+    ProfScope ps(h, QMCB_KERNEL_MOVE, st);
+    launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
     ps.end(st);
     return;
   }
   const dim3 g((cap + h->wpb_move - 1) / h->wpb_move), b(32 * h->wpb_move);
   const size_t sm = h->smem_move;
   ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-  if (h->params.precision == QMCB_PREC_MIXED) {
-    if (extras)
-      launch_move_g<kMetropolis, float, MIXED_TI, true>(h, g, b, sm, st, cfg, slots, num, d_num, R_in, mv, o);
-    else
-      launch_move_g<kMetropolis, float, MIXED_TI, false>(h, g, b, sm, st, cfg, slots, num, d_num, R_in, mv, o);
-  } else {
-    if (extras)
-      launch_move_g<kMetropolis, double, double, true>(h, g, b, sm, st, cfg, slots, num, d_num, R_in, mv, o);
-    else
-      launch_move_g<kMetropolis, double, double, false>(h, g, b, sm, st, cfg, slots, num, d_num, R_in, mv, o);
-  }
+  launch_move_g(h, kMetropolis, h->params.precision == QMCB_PREC_MIXED, extras, g, b, sm, st, cfg, slots, num, d_num,
+                R_in, mv, o);
   ps.end(st);
-}
-
-// The dynamic shared-memory limit of every move-kernel instantiation.
-template <bool kMetropolis, typename TS, typename TI>
-static cudaError_t move_smem_limits(int bytes)
-{
-  cudaError_t e = cudaSuccess;
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_move<kMetropolis, TS, TI, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_move<kMetropolis, TS, TI, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_move<kMetropolis, TS, TI, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_move<kMetropolis, TS, TI, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  return e;
 }
 
 // ---------------------------------------------------------------------------
@@ -585,22 +712,30 @@ static cudaError_t rows_prep_bf_limits(int bytes)
   return e;
 }
 
+// The move kernel's smaller scratch when its rows come from a batched
+// kernel: no basis rows, region A holds only the slice sums and the new
+// drifts (and the three-body partner gradients).
+static void rows_layout(qmcb_handle *h)
+{
+  Layout L = h->lay;
+  const int ra = even(std::max(kPart + 6 * h->N, h->sys.ntb > 0 ? 3 * h->N * h->sys.M : 0));
+  L.mv_stride += ra - L.mv_region_a;
+  L.mv_region_a = ra;
+  h->lay_rows = L;
+  const size_t per_move = sizeof(double) * (size_t)L.mv_stride;
+  h->wpb_rows = best_warps_per_block(h, per_move);
+  h->smem_rows = per_move * h->wpb_rows;
+}
+
 // What every tensor-core rows mode shares, once per handle: the rows
-// buffer, the move kernel's smaller scratch layout (no basis rows), the
-// prep kernels' CTA shapes and shared-memory limits.
+// buffer, the prep kernels' CTA shapes and shared-memory limits.
 static int rows_common_setup(qmcb_handle *h)
 {
   if (h->d_rows_out) return QMCB_OK;
   const int K = h->K, N = h->N;
-  // the move kernel without the basis rows: region A holds only the slice
-  // sums and the new drifts (and the three-body partner gradients)
-  Layout L = h->lay;
-  const int ra = even(std::max(kPart + 6 * N, h->sys.ntb > 0 ? 3 * N * h->sys.M : 0));
-  L.mv_stride += ra - L.mv_region_a;
-  L.mv_region_a = ra;
   int max_optin = 0;
   cudaDeviceGetAttribute(&max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
-  const size_t per_move = sizeof(double) * (size_t)L.mv_stride;
+  const size_t per_move = sizeof(double) * (size_t)h->lay_rows.mv_stride;
   const size_t per_prep = sizeof(double) * (size_t)rows_prep_doubles(N, K, h->sys.nslot);
   if (per_move > (size_t)max_optin || per_prep > (size_t)max_optin || kRowsSmem > max_optin ||
       bf_smem_bytes(2) > max_optin)
@@ -609,9 +744,6 @@ static int rows_common_setup(qmcb_handle *h)
   // a wait inside a contraction kernel that gave up sets ctl[3], which
   // returns with every batch's live count
   CKR(cudaMemsetAsync(h->d_ctl + 3, 0, sizeof(int), h->stream));
-  h->lay_rows = L;
-  h->wpb_rows = best_warps_per_block(h, per_move);
-  h->smem_rows = per_move * h->wpb_rows;
   h->wpb_prep = best_warps_per_block(h, per_prep);
   h->smem_prep = per_prep * h->wpb_prep;
   CKR(rows_prep_limits<true>(max_optin));
@@ -1023,6 +1155,7 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   CKC(upload(&h->d_shell, shells));
   CKC(upload(&h->d_fn, fn));
   CKC(upload(&h->d_xsl, xsl));
+  if (!md) CKC(rows64_tables(h, shells, fn, nuc, pexp, pcoef, ct, nact));
   CKC(upload(&h->d_fq, fq));
   CKC(upload(&h->d_pexp, pexp));
   CKC(upload(&h->d_pcoef, pcoef));
@@ -1222,23 +1355,38 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   h->wpb_full = (int)std::min<size_t>(kMaxWarpsPerBlock, max_optin / per_full);
   h->smem_move = per_move * h->wpb_move;
   h->smem_full = per_full * h->wpb_full;
+  if (!md) rows_layout(h);
+  CKC(rows64_limits());
   const size_t per_refresh = sizeof(double) * (size_t)refresh_scratch_doubles(h->N, h->nmax);
   h->wpb_refresh = best_warps_per_block(h, per_refresh);
   h->smem_refresh = per_refresh * h->wpb_refresh;
   // the dynamic shared-memory limit is a per-kernel, process-wide attribute:
   // raise it to the device maximum once, so handles of different systems
   // (each launching with its own size) never undercut one another
-  CKC((move_smem_limits<true, double, double>(max_optin)));
-  CKC((move_smem_limits<false, double, double>(max_optin)));
-  CKC((move_smem_limits<true, float, MIXED_TI>(max_optin)));
-  CKC((move_smem_limits<false, float, MIXED_TI>(max_optin)));
-  CKC(cudaFuncSetAttribute(k_full<double, double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_full<float, MIXED_TI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_full<double, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_full<float, MIXED_TI, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_full_md, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_move_md<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  CKC(cudaFuncSetAttribute(k_move_md<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
+  for (int k = 0; k < 16; k++)
+    CKC(cudaFuncSetAttribute(move_fn(k & 1, k & 2, k & 4, k & 8), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
+  for (int k = 0; k < 4; k++)
+    CKC(cudaFuncSetAttribute(full_fn(k & 1, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
+  for (const void *fn : {full_md_fn(), move_md_fn(true), move_md_fn(false)})
+    CKC(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
+  // Below one full wave of the fused move kernel (a warp per walker, its
+  // scratch limiting the warps per SM) a step takes one walker's latency, and
+  // a rows launch before it only adds its own (10 to 60 electrons, 64 to 512
+  // walkers: 20-45 us a step fused, 25-55 us in two launches); above it the
+  // batched rows win or tie (4,096 / 16,384 walkers, us a step, fused and in
+  // two launches: 16 electrons 50, 126 and 50, 129; 30 electrons 74, 227 and
+  // 65, 187; 60 electrons 207, 693 and 147, 441).  Above 64 electrons a spin
+  // one warp's contraction is the longer latency at any size (140 and 196
+  // electrons, one walker: 137 and 222 us fused, 128 and 200 in two launches;
+  // 1,024 walkers: 368 and 769, 216 and 478).
+  if (h->r64.nchunk > 0) {
+    int n_sm = 0, per_sm = 0;
+    CKC(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
+    CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, move_fn(true, false, h->extras, h->ginv),
+                                                      32 * h->wpb_move, h->smem_move));
+    h->rows64_from = h->nmax > 64 ? 1 : n_sm * per_sm * h->wpb_move + 1;
+    if (max_walkers >= h->rows64_from) CKC(cudaMalloc(&h->d_rows64, sizeof(double) * (size_t)max_walkers * 5 * h->nmax));
+  }
   // the memsets above ran on the legacy default stream, which does not order
   // against the handle's non-blocking stream: finish them before any work is
   // queued there (a late memset of the control words would zero the live count)
@@ -1257,7 +1405,8 @@ int qmcb_destroy(qmcb_handle *h)
                   h->d_en[0], h->d_en[1], h->d_state,   h->d_live,  h->d_live_tmp, h->d_free, h->d_ctl,
                   h->d_copies, h->d_stats, h->d_dump, h->d_ectl,   h->d_slots, h->d_R,     h->d_out,    h->d_status,
                   h->d_rows_A, h->d_rows_B[0], h->d_rows_B[1], h->d_rows_rs, h->d_rows_cs[0], h->d_rows_cs[1],
-                  h->d_rows_out, h->d_bf_A, h->d_bf_B[0], h->d_bf_B[1]};
+                  h->d_rows_out, h->d_bf_A, h->d_bf_B[0], h->d_bf_B[1], h->d_r64_chunk, h->d_r64_rec,
+                  h->d_r64_ct[0], h->d_r64_ct[1], h->d_rows64};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   for (cudaEvent_t e : h->prof_ev) cudaEventDestroy(e);
@@ -1355,22 +1504,39 @@ static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
 {
   // list entries [0, num) (d_num: device count), grid sized for `cap`;
   // the refresh (do_basis = 0) runs with its smaller per-warp scratch
+  if (do_basis && h->params.precision != QMCB_PREC_MIXED && h->r64.nchunk > 0 && !h->sys.cusp &&
+      (h->N > 4 || cap >= 1024)) {
+    // all electrons' orbital rows into the walker state, then the refresh of
+    // the stored rows (with the caller's positions): 1 / 4,096 walkers, us,
+    // one warp a walker and this way: 3 electrons 24, 71 and 26, 57; 10: 79,
+    // 254 and 42, 116; 30: 301, 1,262 and 96, 455; 100: 5,083, 38,592 and 564,
+    // 7,718.  (The cusp replacement works on rows before they are stored.)
+    for (int sp = 0; sp < 2; sp++)
+      rows64_launch(R64_ALL, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num, R_in, MoveArgs{}, sp,
+                    nullptr);
+    do_basis = 0;
+  }
   const int wpb = do_basis ? h->wpb_full : h->wpb_refresh;
   const dim3 g((cap + wpb - 1) / wpb), b(32 * wpb);
   const size_t sm = do_basis ? h->smem_full : h->smem_refresh;
-  if (h->params.precision == QMCB_PREC_MIXED) {
-    if (h->extras)
-      k_full<float, MIXED_TI, true><<<g, b, sm, st>>>(h->sys, h->lay, cfg, h->d_state, slots, num, d_num, R_in, do_basis, o);
-    else
-      k_full<float, MIXED_TI, false><<<g, b, sm, st>>>(h->sys, h->lay, cfg, h->d_state, slots, num, d_num, R_in, do_basis,
-                                                       o);
-  } else {
-    if (h->extras)
-      k_full<double, double, true><<<g, b, sm, st>>>(h->sys, h->lay, cfg, h->d_state, slots, num, d_num, R_in, do_basis, o);
-    else
-      k_full<double, double, false><<<g, b, sm, st>>>(h->sys, h->lay, cfg, h->d_state, slots, num, d_num, R_in, do_basis,
-                                                      o);
-  }
+  launch_kernel(full_fn(h->params.precision == QMCB_PREC_MIXED, h->extras), g, b, sm, st, h->sys, h->lay, cfg,
+                h->d_state, slots, num, d_num, R_in, do_basis, o);
+}
+
+// The several-determinant kernels.
+static void launch_full_md(qmcb_handle *h, int blocks, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
+                           const int *d_num, const double *R_in, int do_basis, const EvalOut &o)
+{
+  launch_kernel(full_md_fn(), dim3(blocks), dim3(32 * h->wpb_full), h->smem_full, st, h->sys, h->lay, cfg, h->d_state,
+                slots, num, d_num, R_in, do_basis, o);
+}
+
+static void launch_move_md(qmcb_handle *h, bool metropolis, int blocks, cudaStream_t st, const RunCfg &cfg,
+                           const int *slots, int num, const int *d_num, const double *R_in, const MoveArgs &mv,
+                           const EvalOut &o)
+{
+  launch_kernel(move_md_fn(metropolis), dim3(blocks), dim3(32 * h->wpb_move), h->smem_move, st, h->sys, h->lay, cfg,
+                h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
 }
 
 // Device address of a host array that kernels can store into directly:
@@ -1471,15 +1637,12 @@ static int launch_eval(qmcb_handle *h, int which_e, const int *d_slots, int num,
     if (mixed) return fail(h, QMCB_E_ARG, "evaluate: several determinants run in FP64 (precision QMCB_PREC_FP64)");
     if (which_e < 0) {
       int blocks = (num + h->wpb_full - 1) / h->wpb_full;
-      k_full_md<<<blocks, 32 * h->wpb_full, h->smem_full, st>>>(h->sys, h->lay, cfg, h->d_state, d_slots, num,
-                                                                 nullptr, d_R, 1, o);
+      launch_full_md(h, blocks, st, cfg, d_slots, num, nullptr, d_R, 1, o);
     } else {
       MoveArgs mv{which_e, 0, 0, 0};
       mv.rin_moved = rin_moved;
       int blocks = (num + h->wpb_move - 1) / h->wpb_move;
-      k_move_md<false><<<blocks, 32 * h->wpb_move, h->smem_move, st>>>(h->sys, h->lay, cfg, h->d_state, d_slots,
-                                                                        num, nullptr, d_R, mv, h->d_ectl,
-                                                                        h->d_stats, o);
+      launch_move_md(h, false, blocks, st, cfg, d_slots, num, nullptr, d_R, mv, o);
     }
     CK(cudaGetLastError());
     if (which_e < 0) h->state_prec = h->params.precision;
@@ -1671,8 +1834,7 @@ static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *du
     EvalOut o{};
     if (h->md) {
       ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-      k_move_md<true><<<blocks, 32 * h->wpb_move, h->smem_move, st>>>(h->sys, h->lay, cfg, h->d_state, h->d_live, 0,
-                                                                       h->d_ctl, nullptr, mv, h->d_ectl, h->d_stats, o);
+      launch_move_md(h, true, blocks, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o);
       ps.end(st);
     } else {
       launch_move<true>(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o);
@@ -1700,8 +1862,7 @@ static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *du
       EvalOut o2{};
       ProfScope ps(h, QMCB_KERNEL_REFRESH, st);
       if (h->md)
-        k_full_md<<<blocks_full, 32 * h->wpb_full, h->smem_full, st>>>(h->sys, h->lay, cfg, h->d_state, h->d_live, 0,
-                                                                        h->d_ctl, nullptr, 0, o2);
+        launch_full_md(h, blocks_full, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2);
       else
         launch_full(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2);
       ps.end(st);
@@ -2002,21 +2163,6 @@ static bool member_extras(const qmcb_handle *h)
   return h->extras || h->params.sampling == QMCB_UMRIGAR93_IMPORTANCE_SAMPLING;
 }
 
-// Persistent grid of one bucket: as many blocks as fit on every SM at once.
-// The group move kernel for a bucket's flags; cbase >= 0: the group's
-// member table sits in c_gm from cbase on.
-static const void *group_move_fn(bool extras, bool ginv, bool cst, bool md)
-{
-  const void *fns[10] = {
-      (const void *)k_move_group<false, false, false, false>, (const void *)k_move_group<true, false, false, false>,
-      (const void *)k_move_group<false, true, false, false>,  (const void *)k_move_group<true, true, false, false>,
-      (const void *)k_move_group<false, false, true, false>,  (const void *)k_move_group<true, false, true, false>,
-      (const void *)k_move_group<false, true, true, false>,   (const void *)k_move_group<true, true, true, false>,
-      (const void *)k_move_group<true, false, false, true>,   (const void *)k_move_group<true, false, true, true>};
-  if (md) return fns[8 + (cst ? 1 : 0)];
-  return fns[(extras ? 1 : 0) + (ginv ? 2 : 0) + (cst ? 4 : 0)];
-}
-
 // Doubles of shared memory one warp of the member's move kernel uses.
 static int member_stride(const qmcb_handle *h) { return (int)(h->smem_move / sizeof(double) / h->wpb_move); }
 
@@ -2156,14 +2302,14 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
     for (int i = B.first; i < B.first + B.count; i++) dmc |= g->mem[i]->params.run_type == QMCB_DMC;
     const GroupMember *gm = g->d_gm + B.first;
     for (int t = 0; t < n_steps; t++) {
-      // members on tensor-core rows: their step's rows first (one prep and
-      // one contraction launch per member), each member's on its own stream
+      // members on batched rows: their step's rows first (one or two launches
+      // per member), each member's on its own stream
       // so that the members' small kernels overlap, joined back into the
       // bucket's stream before its move kernel
       bool forked = false;
       for (int i = B.first; i < B.first + B.count; i++) {
         qmcb_handle *h = g->mem[i];
-        if (!rows_mode(h->params.precision)) continue;
+        if (!batched_rows(h)) continue;
         if (!forked) {
           GK(cudaEventRecord(g->step_ev[b], sb));
           forked = true;
@@ -2175,18 +2321,18 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
         mv.do_reweight = mv.e == 0;
         mv.reweight_on = mv.step >= h->params.reweight_start_step;
         mv.dump = nullptr;
-        launch_rows<true>(h, h->max_walkers, h->stream, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, mv,
-                          member_extras(h), false);
+        if (rows_mode(h->params.precision))
+          launch_rows<true>(h, h->max_walkers, h->stream, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, mv,
+                            member_extras(h), false);
+        else
+          GK(rows64_launch(R64_PROPOSE, h->sys, h->lay, make_cfg(h->params), h->r64, h->d_state, h->max_walkers,
+                           h->stream, h->d_live, 0, h->d_ctl, nullptr, mv, mv.e < h->sys.na ? 0 : 1, h->d_rows64));
         GK(cudaEventRecord(g->rows_ev[i], h->stream));
         GK(cudaStreamWaitEvent(sb, g->rows_ev[i], 0));
       }
       GK(cudaMemsetAsync(g->d_counter + b, 0, sizeof(int), sb));
       GK(launch_group_move_any(B, sb, gm, t, g->d_counter + b, g->cbase >= 0 ? g->cbase + B.first : -1));
-      if (dmc) {
-        k_branch_group<<<B.count, 1024, 0, sb>>>(gm, t);
-        k_copy_group<<<dim3(64, B.count), 256, 0, sb>>>(gm, t);
-        k_energy_group<<<(B.count + 127) / 128, 128, 0, sb>>>(gm, B.count, t);
-      }
+      if (dmc) group_branch(gm, B.count, t, sb);
       if (refresh) {
         for (int i = B.first; i < B.first + B.count; i++) {
           qmcb_handle *h = g->mem[i];
@@ -2195,9 +2341,7 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
             EvalOut o2{};
             const int blocks_full = (h->max_walkers + h->wpb_full - 1) / h->wpb_full;
             if (h->md)
-              k_full_md<<<blocks_full, 32 * h->wpb_full, h->smem_full, sb>>>(h->sys, h->lay, make_cfg(h->params),
-                                                                              h->d_state, h->d_live, 0, h->d_ctl,
-                                                                              nullptr, 0, o2);
+              launch_full_md(h, blocks_full, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2);
             else
               launch_full(h, h->max_walkers, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2);
           }
@@ -2322,7 +2466,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
       return gfail(g, QMCB_E_ARG, who + ": several determinants run in FP64 only");
     refresh |= h->params.refresh_interval > 0;
     // the rows kernels take the step number as an argument: no graph replay
-    rows_members |= rows_mode(h->params.precision);
+    rows_members |= batched_rows(h);
   }
   cudaSetDevice(g->device);
   // members' tables, parameters and step numbers
@@ -2330,10 +2474,10 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
   for (int i = 0; i < nm; i++) {
     qmcb_handle *h = g->mem[i];
     GroupMember &G = g->h_gm[i];
-    const bool rows = rows_mode(h->params.precision);
+    const bool rows = batched_rows(h);
     G.S = h->sys;
     G.L = rows ? h->lay_rows : h->lay;  // the move kernel on rows needs no basis scratch
-    G.rows = rows ? h->d_rows_out : nullptr;
+    G.rows = !rows ? nullptr : rows_mode(h->params.precision) ? h->d_rows_out : h->d_rows64;
     G.cfg = make_cfg(h->params);
     G.state = h->d_state;
     G.live = h->d_live;
@@ -2363,8 +2507,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
   for (auto *h : g->mem) GK(cudaStreamSynchronize(h->stream));
   GK(cudaMemcpyAsync(g->d_gm, g->h_gm.data(), sizeof(GroupMember) * nm, cudaMemcpyHostToDevice, st));
   if (g->cbase >= 0)
-    GK(cudaMemcpyToSymbolAsync(c_gm, g->h_gm.data(), sizeof(GroupMember) * nm, sizeof(GroupMember) * g->cbase,
-                               cudaMemcpyHostToDevice, st));
+    GK(group_upload_const(g->h_gm.data(), nm, g->cbase, st));
   for (auto *h : g->mem) GK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_RUN_SUM_W, st));
   // configuration: the tuned one, else the next one not yet timed
   int c = g->chosen;
