@@ -264,7 +264,7 @@ def precision_section(args, rank: int):
                 "kernels_ms": {k: round(v["ms"], 3) for k, v in ks.items() if v["launches"]},
                 "final_walkers": st.n_walkers}
         mv = ks["move"]
-        wpl = st.n_moves / max(mv["launches"], 1)  # walkers per move launch
+        wpl = st.n_moves / max(mv["launches"], 1)  # moves per launch
         mode["move_kernel_roofline"] = {
             "bound": "hbm", "algorithmic_bytes_per_walker_move": bytes_per_move(n, N),
             "achieved_gbs": bytes_per_move(n, N) * wpl / (mv["ms"] / mv["launches"] / 1e3) / 1e9,
@@ -735,18 +735,19 @@ def main():
     ensemble = reduce_energy(st.sum_weight, st.sum_weight_energy, st.sum_weight_energy2, st.n_walkers,
                              st.final_weight)
 
-    # roofline of the move kernel (dominant): algorithmic bytes per launch / launch time
+    # roofline of the move kernel (dominant; a launch runs all the steps between
+    # two branchings or refreshes): algorithmic bytes per launch / launch time
     mv = ks["move"]
     avg_ms = mv["ms"] / max(mv["launches"], 1)
-    walkers_per_launch = st.n_moves / max(mv["launches"], 1)
+    moves_per_launch = st.n_moves / max(mv["launches"], 1)
     bpm = bytes_per_move(n, N)
-    achieved = bpm * walkers_per_launch / (avg_ms / 1e3) / 1e9
+    achieved = bpm * moves_per_launch / (avg_ms / 1e3) / 1e9
     peak, peak_kind = read_peaks()
     tr = read_traffic(WORKLOAD)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                "traffic": (tr * walkers_per_launch) if tr is not None else None,
-                "peak_kind": peak_kind, "kernel": "k_move", "algorithmic_bytes_per_walker_move": bpm,
-                "walkers_per_launch": walkers_per_launch, "avg_launch_ms": avg_ms}
+                "traffic": (tr * moves_per_launch) if tr is not None else None,
+                "peak_kind": peak_kind, "kernel": "k_sweep", "algorithmic_bytes_per_walker_move": bpm,
+                "moves_per_launch": moves_per_launch, "avg_launch_ms": avg_ms}
     launches = int(sum(v["launches"] for v in ks.values()))
 
     # end to end through the public API: one qmcb_run_steps call per step, with

@@ -290,7 +290,7 @@ int qmcb_max_walkers(const qmcb_handle *h);
  *   e_local[num]                           localEnergy
  *   pe[num][3]                             potentialEnergy, neEnergy, eeEnergy
  *   status[num]                            QMCB_ST_* bits (wd->singular)
- * Outputs in mapped page-locked memory are stored by the kernel directly;
+ * Outputs in mapped page-locked memory are stored by kernels directly;
  * pageable ones come back by one copy each.  Returns when they are in place.
  */
 int qmcb_evaluate(qmcb_handle *h, int which_e, const int *slots, int num, const double *R,
@@ -309,8 +309,8 @@ int qmcb_evaluate(qmcb_handle *h, int which_e, const int *slots, int num, const 
  * pageable (outputs then come back by one copy each after the kernel);
  * outputs in page-locked memory mapped into the device's address space
  * (cudaMallocHost / cudaHostAlloc, or cudaHostRegister with
- * cudaHostRegisterMapped) are stored by the kernel directly, so their
- * transfer overlaps the evaluation.  Returns when every output is in place.
+ * cudaHostRegisterMapped) are stored by kernels directly, without a copy.
+ * Returns when every output is in place.
  */
 #define QMCB_OUT_PSI 1        /* log_abs_psi[num], sign[num] */
 #define QMCB_OUT_GRAD 2       /* grad[num][N][3] */
@@ -451,12 +451,13 @@ int qmcb_branch(qmcb_handle *h, int step, int *n_live);
 /* Kernel timing: when enabled, qmcb_run_steps records CUDA events around
  * every launch on the handle's stream and accumulates per-kernel totals.
  * out[2*k] = total ms, out[2*k+1] = launches for k = QMCB_KERNEL_*. */
-#define QMCB_KERNEL_MOVE 0
+#define QMCB_KERNEL_MOVE 0 /* one launch per step, or per run of steps between two branchings or refreshes */
 #define QMCB_KERNEL_BRANCH 1
 #define QMCB_KERNEL_COPY 2
 #define QMCB_KERNEL_ENERGY 3
 #define QMCB_KERNEL_REFRESH 4
-#define QMCB_KERNEL_ROWS_PREP 5 /* tensor-core rows modes: proposal, basis values and their operand planes */
+#define QMCB_KERNEL_ROWS_PREP 5 /* tensor-core rows modes: proposal, basis values and their operand planes;
+                                   FP64: the batched orbital rows of a step */
 #define QMCB_KERNEL_ROWS_MMA 6  /* tensor-core rows modes: the tensor-core contraction */
 #define QMCB_KERNEL_COUNT 7
 int qmcb_set_profiling(qmcb_handle *h, int enable);

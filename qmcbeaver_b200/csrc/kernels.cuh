@@ -962,36 +962,27 @@ __device__ __forceinline__ void jastrow_pe_move_warp(const DevSys &S, double *sR
     }
 }
 
+// What one proposed move adds to the call's sums.
+struct MoveTally {
+  double p;          // acceptance probability
+  bool observed;     // the walker's energy is sampled at this step
+  double w, E, d2;   // its weight, energy, squared proposed displacement
+};
+
 // Acceptance (QMCWalker::calculateMoveAcceptanceProbability,
 // QMcBeaver/src/QMCWalker.cpp:1578-1654), DMC reweight (reweight_walker,
 // :1060-1185) and observables (:2096-2123, 2306-2387) of one proposed move.
-// log_ratio = ln|psi'/psi|, negative = the ratio changed sign.  Writes the
-// walker's weight, age and the per-call sums; returns the acceptance.
-template <bool kUmr>
-__device__ __forceinline__ bool metropolis_reweight(const DevSys &S, const RunCfg &cfg, const MoveArgs &mv,
-                                                    const EnergyCtl *ectl, double *stats, double *sc,
-                                                    const double *sc0, int N, int e, const double *Rn,
-                                                    const double ro[3], const double rn[3], const double *mg,
-                                                    double g_fwd, double u_acc, double log_ratio, bool negative,
-                                                    bool bad, double EL, double modratio, double &p_acc)
+// log_ratio = ln|psi'/psi|, negative = the ratio changed sign, log_g =
+// ln G(R' -> R) - ln G(R -> R'); age, w, mo, Eo_L: the walker's age, weight,
+// drift ratio and local energy before the move.  The leader writes the
+// walker's weight and age; returns the acceptance.
+__device__ __forceinline__ bool accept_and_reweight(const RunCfg &cfg, const MoveArgs &mv, const EnergyCtl *ectl,
+                                                    double *sc, bool leader, double age, double w, double mo,
+                                                    double Eo_L, const double ro[3], const double rn[3], double u_acc,
+                                                    double log_ratio, double log_g, bool negative, bool bad, double EL,
+                                                    double modratio, MoveTally &tally)
 {
-  const int lane = lane_id();
-  // G(R' -> R): only electron e moved, the others contribute (dt v'_i)^2
-  double log_g = 0.0;
-  if (kUmr && cfg.sampling == 2) {
-    log_g = umrigar_log_reverse(S, cfg, e, N, Rn, mg, ro) - g_fwd;
-  } else if (cfg.sampling == 1) {
-    double pr = 0.0;
-    for (int t = lane; t < 3 * N; t += 32) {
-      if (cfg.exact_gf && t / 3 != e) continue;
-      const double tt = (t / 3 == e) ? (ro[t - 3 * e] - rn[t - 3 * e] - cfg.dt * mg[t]) : (cfg.dt * mg[t]);
-      pr += tt * tt;
-    }
-    const double g_rev = warp_sum(pr);
-    log_g = -(g_rev - g_fwd) / (2.0 * cfg.dt);
-  }
   double p = exp(2.0 * log_ratio + log_g);
-  const double age = sc0[SC_AGE];
   const double over = age - cfg.old_walker_acceptance;
   if (!isnan(p)) {
     if (over > 500)
@@ -1004,15 +995,14 @@ __device__ __forceinline__ bool metropolis_reweight(const DevSys &S, const RunCf
   if (bad) p = 0.0;
   if (cfg.run_type == 1 && negative) p = 0.0;
   if (p > 1.0) p = 1.0;
-  p_acc = p;
   const bool accept = p > u_acc;
   const double new_age = accept ? 0.0 : age + 1.0;
-  double w = sc0[SC_WEIGHT];
+  tally.p = p;
+  tally.observed = false;
   if (mv.do_reweight) {
     if (cfg.run_type == 1 && mv.reweight_on) {
       const double ET = ectl->e_trial, Eest = ectl->e_est;
-      const double mo = sc0[SC_MODRATIO];
-      double Eo = sc0[SC_EL];
+      double Eo = Eo_L;
       double Et = bad ? Eo : EL;
       if (cfg.ecut == 1) {
         Et *= bad ? mo : modratio;
@@ -1046,11 +1036,11 @@ __device__ __forceinline__ bool metropolis_reweight(const DevSys &S, const RunCf
         w *= 0.9;
       else
         w *= dW;
-      if (lane == 0) sc[SC_DW] = dW;
+      if (leader) sc[SC_DW] = dW;
       if (cfg.deletion) {
         // QMCWalker::reweight_walker's deletions (QMcBeaver/src/QMCWalker.cpp:1196-1365),
         // on the accepted configuration's local energy
-        const double rel = fabs(((accept ? EL : sc0[SC_EL]) - cfg.e_orig) / cfg.e_orig);
+        const double rel = fabs(((accept ? EL : Eo_L) - cfg.e_orig) / cfg.e_orig);
         bool del;
         if (mv.step - cfg.equil_steps < -100)
           del = w > 2.0 * cfg.branching_threshold || w < 0.1 || dW > 1.5 || dW < 0.5 || isnan(dW) ||
@@ -1063,33 +1053,70 @@ __device__ __forceinline__ bool metropolis_reweight(const DevSys &S, const RunCf
       // at the next branching instead of poisoning the ensemble sums
       if (!isfinite(w)) w = 0.0;
     }
-    const double Eobs = p * (bad ? 0.0 : EL) + (1.0 - p) * sc0[SC_EL];
+    const double Eobs = p * (bad ? 0.0 : EL) + (1.0 - p) * Eo_L;
     // rel_cutoff filter of QMCWalker::calculateObservables (QMcBeaver/src/QMCWalker.cpp:2336-2351)
     const bool in_avg = fabs((Eobs - cfg.e_orig) / cfg.e_orig) < cfg.rel_cutoff;
-    if (lane == 0 && w > 0.0 && in_avg) {
-      atomicAdd(&stats[ST_SUM_W], w);
-      atomicAdd(&stats[ST_SUM_WE], w * Eobs);
-      atomicAdd(&stats[ST_SUM_WE2], w * Eobs * Eobs);
-      atomicAdd(&stats[ST_RUN_SUM_W], w);
-      atomicAdd(&stats[ST_RUN_SUM_WE], w * Eobs);
-      atomicAdd(&stats[ST_RUN_COUNT], 1.0);
-      if (cfg.dyn_dt) {
-        // distance the moved electron was proposed to go, as
-        // QMCWalker::calculateObservables samples it (QMcBeaver/src/QMCWalker.cpp:2176-2178, 2376-2383)
-        const double d2 = (rn[0] - ro[0]) * (rn[0] - ro[0]) + (rn[1] - ro[1]) * (rn[1] - ro[1]) +
-                          (rn[2] - ro[2]) * (rn[2] - ro[2]);
-        atomicAdd(&stats[ST_RUN_SUM_WPD2], w * p * d2);
-        atomicAdd(&stats[ST_RUN_SUM_WD2], w * d2);
-      }
-    }
+    tally.observed = w > 0.0 && in_avg;
+    tally.w = w;
+    tally.E = Eobs;
+    // distance the moved electron was proposed to go, as
+    // QMCWalker::calculateObservables samples it (QMcBeaver/src/QMCWalker.cpp:2176-2178, 2376-2383)
+    tally.d2 = (rn[0] - ro[0]) * (rn[0] - ro[0]) + (rn[1] - ro[1]) * (rn[1] - ro[1]) +
+               (rn[2] - ro[2]) * (rn[2] - ro[2]);
   }
-  if (lane == 0) {
-    atomicAdd(&stats[ST_SUM_ACC], p);
-    atomicAdd(&stats[ST_MOVES], 1.0);
-    if (bad) atomicAdd(&stats[ST_SINGULAR], 1.0);
+  if (leader) {
     sc[SC_WEIGHT] = w;
     sc[SC_AGE] = new_age;
     if (accept) sc[SC_AGE_MOVED] = age;
+  }
+  return accept;
+}
+
+// The same for a warp on one walker: the reverse Green's function, then the
+// acceptance, and the sums by atomics.
+template <bool kUmr>
+__device__ __forceinline__ bool metropolis_reweight(const DevSys &S, const RunCfg &cfg, const MoveArgs &mv,
+                                                    const EnergyCtl *ectl, double *stats, double *sc,
+                                                    const double *sc0, int N, int e, const double *Rn,
+                                                    const double ro[3], const double rn[3], const double *mg,
+                                                    double g_fwd, double u_acc, double log_ratio, bool negative,
+                                                    bool bad, double EL, double modratio, double &p_acc)
+{
+  const int lane = lane_id();
+  // G(R' -> R): only electron e moved, the others contribute (dt v'_i)^2
+  double log_g = 0.0;
+  if (kUmr && cfg.sampling == 2) {
+    log_g = umrigar_log_reverse(S, cfg, e, N, Rn, mg, ro) - g_fwd;
+  } else if (cfg.sampling == 1) {
+    double pr = 0.0;
+    for (int t = lane; t < 3 * N; t += 32) {
+      if (cfg.exact_gf && t / 3 != e) continue;
+      const double tt = (t / 3 == e) ? (ro[t - 3 * e] - rn[t - 3 * e] - cfg.dt * mg[t]) : (cfg.dt * mg[t]);
+      pr += tt * tt;
+    }
+    const double g_rev = warp_sum(pr);
+    log_g = -(g_rev - g_fwd) / (2.0 * cfg.dt);
+  }
+  MoveTally ty;
+  const bool accept = accept_and_reweight(cfg, mv, ectl, sc, lane == 0, sc0[SC_AGE], sc0[SC_WEIGHT], sc0[SC_MODRATIO],
+                                          sc0[SC_EL], ro, rn, u_acc, log_ratio, log_g, negative, bad, EL, modratio, ty);
+  p_acc = ty.p;
+  if (lane == 0) {
+    if (ty.observed) {
+      atomicAdd(&stats[ST_SUM_W], ty.w);
+      atomicAdd(&stats[ST_SUM_WE], ty.w * ty.E);
+      atomicAdd(&stats[ST_SUM_WE2], ty.w * ty.E * ty.E);
+      atomicAdd(&stats[ST_RUN_SUM_W], ty.w);
+      atomicAdd(&stats[ST_RUN_SUM_WE], ty.w * ty.E);
+      atomicAdd(&stats[ST_RUN_COUNT], 1.0);
+      if (cfg.dyn_dt) {
+        atomicAdd(&stats[ST_RUN_SUM_WPD2], ty.w * ty.p * ty.d2);
+        atomicAdd(&stats[ST_RUN_SUM_WD2], ty.w * ty.d2);
+      }
+    }
+    atomicAdd(&stats[ST_SUM_ACC], ty.p);
+    atomicAdd(&stats[ST_MOVES], 1.0);
+    if (bad) atomicAdd(&stats[ST_SINGULAR], 1.0);
   }
   return accept;
 }

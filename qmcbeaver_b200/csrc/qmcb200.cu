@@ -27,6 +27,7 @@
 #include "launches.h"
 #include "population.cuh"
 #include "rows64.h"
+#include "sweep.h"
 
 using namespace qmcb;
 
@@ -71,6 +72,7 @@ struct qmcb_handle {
   int rows64_from = INT_MAX;  // FP64 single-electron moves of this many walkers take their rows from k_rows64
   int4 *d_r64_chunk = nullptr;
   double *d_r64_rec = nullptr;
+  bool sweep = false;  // small spins: k_sweep can run the FP64 steps
   double *d_r64_ct[2] = {nullptr, nullptr}, *d_rows64 = nullptr;
   Layout lay_rows{};  // move-kernel scratch without the basis rows
   double *d_pade = nullptr;
@@ -414,7 +416,7 @@ static void launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extr
 // emptiest chunk with room (so that every chunk holds a like mix of cheap and
 // dear shells), sorted by cost within a chunk.  Complete s, p and d shells of
 // at most three primitives take the kernel's fast kinds; any other shell of
-// more than kR64Chunk functions is cut.  r64.nchunk
+// more functions than a chunk holds is cut.  r64.nchunk
 // stays 0 (the kernel is not used) when a shell's record would not fit.
 static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells, const std::vector<int2> &fn,
                                  const std::vector<double4> &nuc, const std::vector<double> &pexp,
@@ -431,6 +433,7 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
     const int nmem = (int)it.members.size();
     return it.kind == kR64Any ? 5 + it.np + nmem * (it.np + 1) : 7 + 3 * nmem;
   };
+  const int cap = rows64_chunk(h->nmax);
   std::vector<Item> items;
   for (const int4 &sh : shells) {
     const int nmem = sh.z & 0xff, L = (sh.z >> 8) & 0xff, np = sh.z >> 16;
@@ -447,9 +450,9 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
         continue;
       }
     }
-    for (int m = 0; m < nmem; m += kR64Chunk) {
+    for (int m = 0; m < nmem; m += cap) {
       it.members.clear();
-      for (int k = m; k < std::min(nmem, m + kR64Chunk); k++) it.members.push_back(sh.y + k);
+      for (int k = m; k < std::min(nmem, m + cap); k++) it.members.push_back(sh.y + k);
       items.push_back(it);
     }
   }
@@ -457,13 +460,14 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
     if (doubles(it) >= kR64RecMax) return cudaSuccess;
   std::stable_sort(items.begin(), items.end(),
                    [](const Item &a, const Item &b) { return a.members.size() > b.members.size(); });
-  std::vector<std::vector<Item>> chunks((h->K + kR64Chunk - 1) / kR64Chunk);
+  std::vector<std::vector<Item>> chunks((h->K + cap - 1) / cap);
   std::vector<int> fill(chunks.size(), 0), size(chunks.size(), 0);
   for (const Item &it : items) {
     const int nmem = (int)it.members.size();
     int best = -1;
     for (size_t c = 0; c < chunks.size(); c++)
-      if (fill[c] + nmem <= kR64Chunk && size[c] + doubles(it) < kR64RecMax && (best < 0 || fill[c] < fill[best]))
+      if (fill[c] + nmem <= cap && size[c] + doubles(it) < kR64RecMax && chunks[c].size() < 16 + 4 * (h->nmax > 16) &&
+          (best < 0 || fill[c] < fill[best]))
         best = (int)c;
     if (best < 0) {
       best = (int)chunks.size();
@@ -551,6 +555,20 @@ static bool rows64_moves(const qmcb_handle *h, int cap)
   return h->params.precision == QMCB_PREC_FP64 && cap >= h->rows64_from;
 }
 
+// Whether k_sweep runs the FP64 moves: at every size (us a step, 1 / 512 /
+// 4,096 / 16,384 walkers: 6 electrons 9, 9, 11, 26 against 18, 19, 42, 107 by
+// the move kernel; 30 electrons 17, 20, 27, 98 against 28, 27, 74, 227).  It
+// has no cusp replacement, three-body terms or Umrigar93 moves.
+static bool sweep_moves(const qmcb_handle *h)
+{
+  return h->sweep && h->params.precision == QMCB_PREC_FP64;
+}
+
+static bool sweep_steps(const qmcb_handle *h)
+{
+  return sweep_moves(h) && h->params.sampling != QMCB_UMRIGAR93_IMPORTANCE_SAMPLING;
+}
+
 // Whether the steps of all a handle's walkers take rows from a batched kernel.
 static bool batched_rows(const qmcb_handle *h)
 {
@@ -625,6 +643,16 @@ template <bool kMetropolis>
 static void launch_move(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
                         const int *d_num, const double *R_in, MoveArgs mv, EvalOut o)
 {
+  if (!kMetropolis && sweep_moves(h)) {
+    SweepArgs a{};
+    a.e = mv.e;
+    a.rin_moved = mv.rin_moved;
+    ProfScope ps(h, QMCB_KERNEL_MOVE, st);
+    sweep_launch(false, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num, R_in, a, h->d_ectl,
+                 h->d_stats, o);
+    ps.end(st);
+    return;
+  }
   // the Umrigar93 move is compiled only into the extras instantiation
   const bool extras = h->extras || (kMetropolis && cfg.sampling == QMCB_UMRIGAR93_IMPORTANCE_SAMPLING);
   if (rows_mode(h->params.precision)) {
@@ -1380,6 +1408,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   // electrons, one walker: 137 and 222 us fused, 128 and 200 in two launches;
   // 1,024 walkers: 368 and 769, 216 and 478).
   if (h->r64.nchunk > 0) {
+    CKC(sweep_limits(max_optin));
+    h->sweep = h->nmax <= kSweepMax && !h->extras && !h->ginv && sweep_smem_bytes(h->nmax, h->lay, h->r64) <= max_optin;
     int n_sm = 0, per_sm = 0;
     CKC(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
     CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, move_fn(true, false, h->extras, h->ginv),
@@ -1554,21 +1584,23 @@ static void *mapped_device_ptr(void *p)
   return a.type == cudaMemoryTypeHost ? a.devicePointer : nullptr;
 }
 
-// Destinations of the evaluate outputs.  The per-electron arrays (grad,
-// mod_grad) go straight into the caller's array when that array is
-// page-locked and mapped: the kernel's stores of a walker's 3N values cross
-// the bus while it runs.  The per-walker values (psi, sign, lap, E_L,
-// potentials, status) always go to the handle's device buffer first; after
-// the kernel, one k_put_outputs launch moves the ones whose host arrays are
-// mapped in full packets, and one copy each brings back the rest (pageable
-// arrays).  Outputs not selected are not written at all.
+// Destinations of the evaluate outputs.  The per-walker values (psi, sign,
+// lap, E_L, potentials, status) go to the handle's device buffer; after the
+// kernel, one k_put_outputs launch moves the ones whose host arrays are
+// page-locked and mapped in full packets, and one copy each brings back the
+// rest (pageable arrays).  The per-electron arrays (grad, mod_grad) go the same
+// way when the sweep kernel runs the move, and else (direct) straight into a
+// mapped array, the stores crossing the bus while the kernel runs: 4,096
+// walkers of 30 electrons, us a call, stored directly and by k_put_outputs,
+// sweep kernel 210 and 199, move kernel 209 and 229.  Outputs not selected are
+// not written at all.
 struct EvalDst {
   void *host[8], *dev[8], *kernel[8];
   size_t bytes[8];
   bool mapped[8];
 };
 
-static EvalOut eval_destinations(qmcb_handle *h, int num, unsigned mask, double *log_abs_psi, double *sign,
+static EvalOut eval_destinations(qmcb_handle *h, bool direct, int num, unsigned mask, double *log_abs_psi, double *sign,
                                  double *grad, double *mod_grad, double *lap, double *e_local, double *pe,
                                  unsigned char *status, EvalDst &d)
 {
@@ -1592,8 +1624,7 @@ static EvalOut eval_destinations(qmcb_handle *h, int num, unsigned mask, double 
       void *m = mapped_device_ptr(host[i]);
       d.mapped[i] = m != nullptr;
       if (m) d.host[i] = m;
-      const bool per_electron = i == 2 || i == 3;
-      d.kernel[i] = (m && per_electron) ? m : dev[i];
+      d.kernel[i] = m && direct && (i == 2 || i == 3) ? m : dev[i];
     }
   }
   return EvalOut{(double *)d.kernel[0], (double *)d.kernel[1], (double *)d.kernel[2], (double *)d.kernel[3],
@@ -1696,7 +1727,7 @@ int qmcb_evaluate(qmcb_handle *h, int which_e, const int *slots, int num, const 
   CK(cudaMemcpyAsync(h->d_R, R, sizeof(double) * (size_t)num * 3 * N, cudaMemcpyHostToDevice, st));
   // every non-NULL output is returned
   EvalDst dst;
-  const EvalOut o = eval_destinations(h, num, QMCB_OUT_ALL, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
+  const EvalOut o = eval_destinations(h, which_e < 0 || !sweep_moves(h), num, QMCB_OUT_ALL, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
                                       status, dst);
   int rc = launch_eval(h, which_e, h->d_slots, num, h->d_R, o, st);
   if (rc) return rc;
@@ -1731,7 +1762,7 @@ int qmcb_evaluate_moved(qmcb_handle *h, int which_e, const int *slots, int num, 
   CK(cudaMemcpyAsync(h->d_slots, slots, sizeof(int) * num, cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(h->d_R, r_moved, sizeof(double) * 3 * (size_t)num, cudaMemcpyHostToDevice, st));
   EvalDst dst;
-  const EvalOut o = eval_destinations(h, num, out_mask, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
+  const EvalOut o = eval_destinations(h, !sweep_moves(h), num, out_mask, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
                                       status, dst);
   int rc = launch_eval(h, which_e, h->d_slots, num, h->d_R, o, st, 1);
   if (rc) return rc;
@@ -1804,25 +1835,13 @@ int qmcb_init_walkers(qmcb_handle *h, int n, const double *R)
   return QMCB_OK;
 }
 
-// Enqueues n_steps Monte Carlo steps and the copy of the step statistics
-// into the handle's pinned buffer, then records the completion event.
-// dump: device buffer for the configuration records of every step's move
-// (each step overwrites it; null: none).
-static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *dump = nullptr)
+// The launches of n_steps Monte Carlo steps on st (dump: see enqueue_steps).
+static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int first_step, int n_steps, double *dump)
 {
-  if (n_steps < 0 || first_step < 0) return fail(h, QMCB_E_ARG, "qmcb_run_steps: bad step range");
-  if (!h->evaluated_once) return fail(h, QMCB_E_STATE, "qmcb_run_steps: call qmcb_init_walkers first");
-  if (h->state_prec != state_kind(h->params.precision))
-    return fail(h, QMCB_E_STATE, "qmcb_run_steps: walker state was written in another precision; call qmcb_init_walkers");
-  if (h->n_flight >= 2) return fail(h, QMCB_E_STATE, "qmcb_run_steps_async: two batches of steps are already in flight on this handle");
-  if (h->n_live_host <= 0) return fail(h, QMCB_E_STATE, "qmcb_run_steps: no live walkers (population died out)");
-  cudaStream_t st = h->stream;
-  RunCfg cfg = make_cfg(h->params);
-  // per-call sums; the running E_est sums persist across calls
-  CK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_RUN_SUM_W, st));
   const int blocks = (h->max_walkers + h->wpb_move - 1) / h->wpb_move;
   const int blocks_full = (h->max_walkers + h->wpb_full - 1) / h->wpb_full;
   const bool dmc = h->params.run_type == QMCB_DMC;
+  const bool sweep = sweep_steps(h);
   for (int s = 0; s < n_steps; s++) {
     int step = first_step + s;
     MoveArgs mv;
@@ -1832,7 +1851,22 @@ static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *du
     mv.reweight_on = step >= h->params.reweight_start_step;
     mv.dump = dump;
     EvalOut o{};
-    if (h->md) {
+    if (sweep) {
+      // all steps up to the next branching or refresh in one launch
+      SweepArgs a{};
+      a.step0 = step;
+      a.dump = dump;
+      a.reweight_start = h->params.reweight_start_step;
+      const int refresh = h->params.refresh_interval;
+      for (a.nsteps = 1; s + 1 < n_steps && !(dmc && step % h->N == 0) && !(refresh > 0 && (step + 1) % refresh == 0);
+           a.nsteps++, s++)
+        step++;
+      mv.e = step % h->N;
+      ProfScope ps(h, QMCB_KERNEL_MOVE, st);
+      CK(sweep_launch(true, h->sys, h->lay, cfg, h->r64, h->d_state, h->max_walkers, st, h->d_live, 0, h->d_ctl,
+                      nullptr, a, h->d_ectl, h->d_stats, o));
+      ps.end(st);
+    } else if (h->md) {
       ProfScope ps(h, QMCB_KERNEL_MOVE, st);
       launch_move_md(h, true, blocks, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o);
       ps.end(st);
@@ -1869,6 +1903,27 @@ static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *du
     }
   }
   CK(cudaGetLastError());
+  return QMCB_OK;
+}
+
+// Enqueues n_steps Monte Carlo steps and the copy of the step statistics
+// into the handle's pinned buffer, then records the completion event.
+// dump: device buffer for the configuration records of every step's move
+// (each step overwrites it; null: none).
+static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *dump = nullptr)
+{
+  if (n_steps < 0 || first_step < 0) return fail(h, QMCB_E_ARG, "qmcb_run_steps: bad step range");
+  if (!h->evaluated_once) return fail(h, QMCB_E_STATE, "qmcb_run_steps: call qmcb_init_walkers first");
+  if (h->state_prec != state_kind(h->params.precision))
+    return fail(h, QMCB_E_STATE, "qmcb_run_steps: walker state was written in another precision; call qmcb_init_walkers");
+  if (h->n_flight >= 2) return fail(h, QMCB_E_STATE, "qmcb_run_steps_async: two batches of steps are already in flight on this handle");
+  if (h->n_live_host <= 0) return fail(h, QMCB_E_STATE, "qmcb_run_steps: no live walkers (population died out)");
+  cudaStream_t st = h->stream;
+  RunCfg cfg = make_cfg(h->params);
+  // per-call sums; the running E_est sums persist across calls
+  CK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_RUN_SUM_W, st));
+  const int rc = launch_steps(h, st, cfg, first_step, n_steps, dump);
+  if (rc) return rc;
   const int slot = (h->head + h->n_flight) & 1;
   CK(cudaMemcpyAsync(h->h_stats + slot * ST_COUNT, h->d_stats, sizeof(double) * ST_COUNT, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(h->h_ctl + slot * 4, h->d_ctl, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
@@ -2137,8 +2192,14 @@ struct qmcb_group {
   // own stream, forked from its bucket's stream (step_ev[bucket]) and joined
   // back before the bucket's move kernel (rows_ev[member])
   std::vector<cudaEvent_t> step_ev, rows_ev;
+  // members the sweep kernel steps run beside the buckets, on their own
+  // streams (sweep_ev[member]); the buckets' kernels see them without walkers
+  std::vector<char> sweeps;
+  std::vector<cudaEvent_t> sweep_ev;
+  int *d_no_walkers = nullptr;  // control words of an empty walker list
   cudaGraphExec_t gexec = nullptr;  // the last batch's launch sequence
   int g_steps = -1, g_config = -1;
+  std::vector<char> g_sweeps;
   std::string err;
 };
 
@@ -2296,10 +2357,13 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
   GK(cudaEventRecord(g->fork_ev, st));
   for (size_t b = 0; b < bs.size(); b++) {
     const auto &B = bs[b];
+    bool any = false;
+    for (int i = B.first; i < B.first + B.count; i++) any |= !g->sweeps[i];
+    if (!any) continue;
     cudaStream_t sb = g->side[b];
     GK(cudaStreamWaitEvent(sb, g->fork_ev, 0));
     bool dmc = false;
-    for (int i = B.first; i < B.first + B.count; i++) dmc |= g->mem[i]->params.run_type == QMCB_DMC;
+    for (int i = B.first; i < B.first + B.count; i++) dmc |= !g->sweeps[i] && g->mem[i]->params.run_type == QMCB_DMC;
     const GroupMember *gm = g->d_gm + B.first;
     for (int t = 0; t < n_steps; t++) {
       // members on batched rows: their step's rows first (one or two launches
@@ -2309,7 +2373,7 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
       bool forked = false;
       for (int i = B.first; i < B.first + B.count; i++) {
         qmcb_handle *h = g->mem[i];
-        if (!batched_rows(h)) continue;
+        if (g->sweeps[i] || !batched_rows(h)) continue;
         if (!forked) {
           GK(cudaEventRecord(g->step_ev[b], sb));
           forked = true;
@@ -2336,6 +2400,7 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
       if (refresh) {
         for (int i = B.first; i < B.first + B.count; i++) {
           qmcb_handle *h = g->mem[i];
+          if (g->sweeps[i]) continue;
           const int step = first_steps[g->user[i]] + t;
           if (h->params.refresh_interval > 0 && (step + 1) % h->params.refresh_interval == 0) {
             EvalOut o2{};
@@ -2392,6 +2457,10 @@ int qmcb_group_create(qmcb_handle *const *members, int n, qmcb_group **out)
   cudaError_t e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&g->d_gm, sizeof(GroupMember) * n);
   if (e == cudaSuccess) e = cudaMalloc(&g->d_counter, sizeof(int) * (n + 1));
+  if (e == cudaSuccess) e = cudaMalloc(&g->d_no_walkers, sizeof(int) * 4);
+  if (e == cudaSuccess) e = cudaMemset(g->d_no_walkers, 0, sizeof(int) * 4);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  g->sweep_ev.assign(n, nullptr);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev1);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&g->fork_ev, cudaEventDisableTiming);
@@ -2432,12 +2501,15 @@ int qmcb_group_destroy(qmcb_group *g)
   if (g->gexec) cudaGraphExecDestroy(g->gexec);
   if (g->d_gm) cudaFree(g->d_gm);
   if (g->d_counter) cudaFree(g->d_counter);
+  if (g->d_no_walkers) cudaFree(g->d_no_walkers);
   if (g->ev0) cudaEventDestroy(g->ev0);
   if (g->ev1) cudaEventDestroy(g->ev1);
   if (g->fork_ev) cudaEventDestroy(g->fork_ev);
   for (cudaEvent_t e : g->side_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : g->step_ev) cudaEventDestroy(e);
   for (cudaEvent_t e : g->rows_ev) cudaEventDestroy(e);
+  for (cudaEvent_t e : g->sweep_ev)
+    if (e) cudaEventDestroy(e);
   for (cudaStream_t s2 : g->side) {
     cudaStreamSynchronize(s2);
     cudaStreamDestroy(s2);
@@ -2453,7 +2525,8 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
 {
   if (!g || !first_steps || n_steps < 0) return gfail(g, QMCB_E_ARG, "qmcb_group_run_steps: bad argument");
   const int nm = (int)g->mem.size();
-  bool refresh = false, rows_members = false;
+  bool refresh = false, rows_members = false, others = false;
+  g->sweeps.assign(nm, 0);
   for (int i = 0; i < nm; i++) {
     qmcb_handle *h = g->mem[i];
     const std::string who = "qmcb_group_run_steps: member " + std::to_string(g->user[i]);
@@ -2464,6 +2537,9 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
       return gfail(g, QMCB_E_ARG, who + ": groups step FP64 walkers (FP64 or tensor-core orbital rows) only");
     if (h->md && h->params.precision != QMCB_PREC_FP64)
       return gfail(g, QMCB_E_ARG, who + ": several determinants run in FP64 only");
+    g->sweeps[i] = sweep_steps(h);
+    if (g->sweeps[i]) continue;
+    others = true;
     refresh |= h->params.refresh_interval > 0;
     // the rows kernels take the step number as an argument: no graph replay
     rows_members |= batched_rows(h);
@@ -2474,7 +2550,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
   for (int i = 0; i < nm; i++) {
     qmcb_handle *h = g->mem[i];
     GroupMember &G = g->h_gm[i];
-    const bool rows = batched_rows(h);
+    const bool rows = !g->sweeps[i] && batched_rows(h);
     G.S = h->sys;
     G.L = rows ? h->lay_rows : h->lay;  // the move kernel on rows needs no basis scratch
     G.rows = !rows ? nullptr : rows_mode(h->params.precision) ? h->d_rows_out : h->d_rows64;
@@ -2483,13 +2559,13 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     G.live = h->d_live;
     G.live_tmp = h->d_live_tmp;
     G.free_stack = h->d_free;
-    G.ctl = h->d_ctl;
+    G.ctl = g->sweeps[i] ? g->d_no_walkers : h->d_ctl;
     G.copies = h->d_copies;
     G.ectl = h->d_ectl;
     G.stats = h->d_stats;
     G.step0 = first_steps[g->user[i]];
     G.reweight_start = h->params.reweight_start_step;
-    G.dmc = h->params.run_type == QMCB_DMC;
+    G.dmc = !g->sweeps[i] && h->params.run_type == QMCB_DMC;
     G.limit_branching = h->params.limit_branching;
     G.thr_split = h->params.branching_threshold;
     G.thr_fuse = h->params.fusion_threshold;
@@ -2518,8 +2594,19 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
         break;
       }
   GK(cudaEventRecord(g->ev0, st));
-  if (!refresh && !rows_members && n_steps > 0) {
-    if (!(g->gexec && g->g_steps == n_steps && g->g_config == c)) {
+  for (int i = 0; i < nm; i++) {
+    if (!g->sweeps[i]) continue;
+    qmcb_handle *h = g->mem[i];
+    GK(cudaStreamWaitEvent(h->stream, g->ev0, 0));
+    const int rc = launch_steps(h, h->stream, make_cfg(h->params), first_steps[g->user[i]], n_steps, nullptr);
+    if (rc) return gfail(g, rc, "qmcb_group_run_steps: member " + std::to_string(g->user[i]) + ": " + h->err);
+    if (!g->sweep_ev[i]) GK(cudaEventCreateWithFlags(&g->sweep_ev[i], cudaEventDisableTiming));
+    GK(cudaEventRecord(g->sweep_ev[i], h->stream));
+  }
+  if (!others) {
+    // every member runs on its own stream
+  } else if (!refresh && !rows_members && n_steps > 0) {
+    if (!(g->gexec && g->g_steps == n_steps && g->g_config == c && g->g_sweeps == g->sweeps)) {
       if (g->gexec) {
         cudaGraphExecDestroy(g->gexec);
         g->gexec = nullptr;
@@ -2541,12 +2628,15 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
       }
       g->g_steps = n_steps;
       g->g_config = c;
+      g->g_sweeps = g->sweeps;
     }
     GK(cudaGraphLaunch(g->gexec, st));
   } else {
     int rc = group_enqueue(g, c, n_steps, first_steps, refresh);
     if (rc) return rc;
   }
+  for (int i = 0; i < nm; i++)
+    if (g->sweeps[i]) GK(cudaStreamWaitEvent(st, g->sweep_ev[i], 0));
   GK(cudaEventRecord(g->ev1, st));
   for (auto *h : g->mem) {
     GK(cudaMemcpyAsync(h->h_stats, h->d_stats, sizeof(double) * ST_COUNT, cudaMemcpyDeviceToHost, st));

@@ -9,9 +9,14 @@ constexpr int kR64Walkers = 32;              // walkers per CTA: one per lane
 constexpr int kR64Rows = 5 * kR64Walkers;    // row = quantity * 32 + walker
 constexpr int kR64MTiles = kR64Rows / 16;    // 16-row MMA tiles
 constexpr int kR64Chunk = 48;                // basis functions per shared-memory chunk (multiple of 8)
+// Functions per chunk of a handle's tables (nmax: the larger spin).  The
+// sweep kernel (spins of up to 16) keeps two CTAs of 16 walkers per SM with 40,
+// four with 24 (spins of up to 8).
+__host__ __device__ constexpr int rows64_chunk(int nmax) { return nmax <= 8 ? 24 : nmax <= 16 ? 40 : kR64Chunk; }
 // row pitches of the two shared arrays, 4 mod 8 doubles: the 16 lanes of a
 // half-warp fragment load (4 k x 4 columns) then fall on 16 distinct banks
-constexpr int kR64LdA = kR64Rows + 4;
+__host__ __device__ constexpr int rows64_pitch(int walkers) { return 5 * walkers + 4; }
+constexpr int kR64LdA = rows64_pitch(kR64Walkers);
 constexpr int kR64WarpTiles = 4;             // 8-orbital tiles per warp (accumulators: 4 x 4 doubles per lane)
 constexpr int kR64TilesMax = 2 * kR64WarpTiles;  // 8-orbital tiles per CTA
 
