@@ -506,7 +506,8 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
     }
     // stored Slater rows in the state precision TS; the basis, LU and ratio
     // sums here always run in FP64 (this is the refresh of the mixed path)
-    TS *Dv = (TS *)(blk + L.Dv[sp]), *DgT = (TS *)(blk + L.DgT[sp]), *DlT = (TS *)(blk + L.DlT[sp]);
+    TS *Dv = (TS *)(blk + L.Dv[sp]);
+    Deriv4<TS> *D4 = (Deriv4<TS> *)(blk + L.D4[sp]);
     if (do_basis) {
       for (int e = 0; e < n; e++) {
         double r[3] = {Rs[3 * (base + e)], Rs[3 * (base + e) + 1], Rs[3 * (base + e) + 2]};
@@ -520,10 +521,7 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
         }
         for (int o = lane; o < n; o += 32) {
           Dv[e * n + o] = (TS)Dn[o];
-          DgT[(0 * n + o) * n + e] = (TS)Dn[n + o];
-          DgT[(1 * n + o) * n + e] = (TS)Dn[2 * n + o];
-          DgT[(2 * n + o) * n + e] = (TS)Dn[3 * n + o];
-          DlT[o * n + e] = (TS)Dn[4 * n + o];
+          D4[o * n + e] = {(TS)Dn[n + o], (TS)Dn[2 * n + o], (TS)Dn[3 * n + o], (TS)Dn[4 * n + o]};
         }
         __syncwarp();
       }
@@ -541,10 +539,11 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
       double gx = 0, gy = 0, gz = 0;
       for (int o = 0; o < n; o++) {
         double iv = X[o * n + e];
-        lp += (double)DlT[o * n + e] * iv;
-        gx += (double)DgT[(0 * n + o) * n + e] * iv;
-        gy += (double)DgT[(1 * n + o) * n + e] * iv;
-        gz += (double)DgT[(2 * n + o) * n + e] * iv;
+        const Deriv4<TS> g = ld_deriv<true>(&D4[o * n + e]);
+        lp += (double)g.l * iv;
+        gx += (double)g.x * iv;
+        gy += (double)g.y * iv;
+        gz += (double)g.z * iv;
       }
       blk[L.gradD + 3 * (base + e)] = gx;
       blk[L.gradD + 3 * (base + e) + 1] = gy;
@@ -1197,8 +1196,7 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
   double *Ux = sT + (L.Ux - L.gradD);  // grad ln J, updated in place
   const double *mgo = sT + (L.mgrad - L.gradD);
   const double *sc0 = sT + (L.sc - L.gradD);
-  const TS *DgT = (const TS *)(blk + L.DgT[sp]);  // read once per move by the ratio sums
-  const TS *DlT = (const TS *)(blk + L.DlT[sp]);
+  const Deriv4<TS> *D4 = (const Deriv4<TS> *)(blk + L.D4[sp]);  // read once per move by the ratio sums
   double *sc = blk + L.sc;
   const int inv_d = even((n * n * (int)sizeof(TI) + 7) / 8);
   // L2 policies of the HBM-kept inverse (kGInv): kept between its two reads
@@ -1301,32 +1299,27 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
       int r = 0;
       for (; r + kB <= n; r += kB) {
         TI ie[kB], x[kB];
-        TS g0[kB], g1[kB], g2[kB], gl[kB];
+        Deriv4<TS> g[kB];
 #pragma unroll
         for (int u = 0; u < kB; u++) {
           ie[u] = ginv_ld(&InvO[(r + u) * n + el], drop);
           x[u] = ginv_ld(&InvO[(r + u) * n + c], drop);
-          if (c == el) {
-            g0[u] = Dn[n + r + u];
-            g1[u] = Dn[2 * n + r + u];
-            g2[u] = Dn[3 * n + r + u];
-            gl[u] = Dn[4 * n + r + u];
-          } else {
-            g0[u] = __ldcs(&DgT[(0 * n + r + u) * n + c]);
-            g1[u] = __ldcs(&DgT[(1 * n + r + u) * n + c]);
-            g2[u] = __ldcs(&DgT[(2 * n + r + u) * n + c]);
-            gl[u] = __ldcs(&DlT[(r + u) * n + c]);
-          }
+          g[u] = ld_deriv<true>(&D4[(r + u) * n + c]);
+        }
+        if (c == el) {
+#pragma unroll
+          for (int u = 0; u < kB; u++)
+            g[u] = {Dn[n + r + u], Dn[2 * n + r + u], Dn[3 * n + r + u], Dn[4 * n + r + u]};
         }
 #pragma unroll
         for (int u = 0; u < kB; u++) {
           const TI nv = c == el ? (TI)(ie[u] * q) : x[u] - vc * ie[u];
           ginv_st(&Inv[(r + u) * n + c], nv, drop);
           const double iv = (double)nv;
-          gx = fma((double)g0[u], iv, gx);
-          gy = fma((double)g1[u], iv, gy);
-          gz = fma((double)g2[u], iv, gz);
-          ll = fma((double)gl[u], iv, ll);
+          gx = fma((double)g[u].x, iv, gx);
+          gy = fma((double)g[u].y, iv, gy);
+          gz = fma((double)g[u].z, iv, gz);
+          ll = fma((double)g[u].l, iv, ll);
         }
       }
       for (; r < n; r++) {
@@ -1334,17 +1327,12 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
         const TI nv = c == el ? (TI)(ie * q) : ginv_ld(&InvO[r * n + c], drop) - vc * ie;
         ginv_st(&Inv[r * n + c], nv, drop);
         const double iv = (double)nv;
-        if (c == el) {
-          gx = fma((double)Dn[n + r], iv, gx);
-          gy = fma((double)Dn[2 * n + r], iv, gy);
-          gz = fma((double)Dn[3 * n + r], iv, gz);
-          ll = fma((double)Dn[4 * n + r], iv, ll);
-        } else {
-          gx = fma((double)__ldcs(&DgT[(0 * n + r) * n + c]), iv, gx);
-          gy = fma((double)__ldcs(&DgT[(1 * n + r) * n + c]), iv, gy);
-          gz = fma((double)__ldcs(&DgT[(2 * n + r) * n + c]), iv, gz);
-          ll = fma((double)__ldcs(&DlT[r * n + c]), iv, ll);
-        }
+        Deriv4<TS> g = ld_deriv<true>(&D4[r * n + c]);
+        if (c == el) g = {Dn[n + r], Dn[2 * n + r], Dn[3 * n + r], Dn[4 * n + r]};
+        gx = fma((double)g.x, iv, gx);
+        gy = fma((double)g.y, iv, gy);
+        gz = fma((double)g.z, iv, gz);
+        ll = fma((double)g.l, iv, ll);
       }
       lp += ll;
       gD[3 * (base + c)] = gx;
@@ -1392,29 +1380,25 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
         // tables keep the L1
         int o = oa;
         for (; o + 4 <= ob; o += 4) {
-          TS g0[4], g1[4], g2[4], gl[4];
+          Deriv4<TS> g[4];
 #pragma unroll
-          for (int u = 0; u < 4; u++) {
-            g0[u] = __ldcs(&DgT[(0 * n + o + u) * n + e2]);
-            g1[u] = __ldcs(&DgT[(1 * n + o + u) * n + e2]);
-            g2[u] = __ldcs(&DgT[(2 * n + o + u) * n + e2]);
-            gl[u] = __ldcs(&DlT[(o + u) * n + e2]);
-          }
+          for (int u = 0; u < 4; u++) g[u] = ld_deriv<true>(&D4[(o + u) * n + e2]);
 #pragma unroll
           for (int u = 0; u < 4; u++) {
             const double iv = (double)Inv[(o + u) * n + e2];
-            gx = fma((double)g0[u], iv, gx);
-            gy = fma((double)g1[u], iv, gy);
-            gz = fma((double)g2[u], iv, gz);
-            ll = fma((double)gl[u], iv, ll);
+            gx = fma((double)g[u].x, iv, gx);
+            gy = fma((double)g[u].y, iv, gy);
+            gz = fma((double)g[u].z, iv, gz);
+            ll = fma((double)g[u].l, iv, ll);
           }
         }
         for (; o < ob; o++) {
           const double iv = (double)Inv[o * n + e2];
-          gx = fma((double)__ldcs(&DgT[(0 * n + o) * n + e2]), iv, gx);
-          gy = fma((double)__ldcs(&DgT[(1 * n + o) * n + e2]), iv, gy);
-          gz = fma((double)__ldcs(&DgT[(2 * n + o) * n + e2]), iv, gz);
-          ll = fma((double)__ldcs(&DlT[o * n + e2]), iv, ll);
+          const Deriv4<TS> g = ld_deriv<true>(&D4[o * n + e2]);
+          gx = fma((double)g.x, iv, gx);
+          gy = fma((double)g.y, iv, gy);
+          gz = fma((double)g.z, iv, gz);
+          ll = fma((double)g.l, iv, ll);
         }
       }
       lp += ll;
@@ -1498,13 +1482,11 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
     } else if (lane == 0) {
       sc[SC_INVCUR_A + sp] = (double)(1 - icur);
     }
-    TS *Dv = (TS *)(blk + L.Dv[sp]), *DgW = (TS *)(blk + L.DgT[sp]), *DlW = (TS *)(blk + L.DlT[sp]);
+    TS *Dv = (TS *)(blk + L.Dv[sp]);
+    Deriv4<TS> *DW = (Deriv4<TS> *)(blk + L.D4[sp]);
     for (int o = lane; o < n; o += 32) {
       Dv[el * n + o] = Dn[o];
-      DgW[(0 * n + o) * n + el] = Dn[n + o];
-      DgW[(1 * n + o) * n + el] = Dn[2 * n + o];
-      DgW[(2 * n + o) * n + el] = Dn[3 * n + o];
-      DlW[o * n + el] = Dn[4 * n + o];
+      DW[o * n + el] = {Dn[n + o], Dn[2 * n + o], Dn[3 * n + o], Dn[4 * n + o]};
     }
     for (int t = lane; t < 3 * n; t += 32) blk[L.gradD + 3 * base + t] = gD[3 * base + t];
     for (int t = lane; t < 3 * N; t += 32) {

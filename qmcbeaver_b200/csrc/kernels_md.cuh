@@ -198,7 +198,7 @@ __device__ __forceinline__ void md_move_walker(const DevSys &S, const Layout &L,
   const double *mgo = sT + (L.mgrad - L.gradD);
   const double *sc0 = sT + (L.sc - L.gradD);
   double *sc = blk + L.sc;
-  const double *DgT = blk + L.DgT[sp], *DlT = blk + L.DlT[sp];
+  const Deriv4<double> *D4 = (const Deriv4<double> *)(blk + L.D4[sp]);
 
   for (int t = lane; t < 3 * N; t += 32) sR[t] = blk[L.R + t];
   for (int t = lane; t < tail; t += 32) sT[t] = blk[L.gradD + t];
@@ -287,10 +287,11 @@ __device__ __forceinline__ void md_move_walker(const DevSys &S, const Layout &L,
         gz = fma(Dn[3 * a + orb], iv, gz);
         lp = fma(Dn[4 * a + orb], iv, lp);
       } else {
-        gx = fma(DgT[(0 * a + orb) * n + e2], iv, gx);
-        gy = fma(DgT[(1 * a + orb) * n + e2], iv, gy);
-        gz = fma(DgT[(2 * a + orb) * n + e2], iv, gz);
-        lp = fma(DlT[orb * n + e2], iv, lp);
+        const Deriv4<double> v = D4[orb * n + e2];
+        gx = fma(v.x, iv, gx);
+        gy = fma(v.y, iv, gy);
+        gz = fma(v.z, iv, gz);
+        lp = fma(v.l, iv, lp);
       }
     }
     double *g = dst.g + ((size_t)c * n + e2) * 3;
@@ -343,13 +344,11 @@ __device__ __forceinline__ void md_move_walker(const DevSys &S, const Layout &L,
   if (accept) {
     double *Rw = blk + L.R;
     if (lane < 3) Rw[3 * e + lane] = rn[lane];
-    double *Dv = blk + L.Dv[sp], *DgW = blk + L.DgT[sp], *DlW = blk + L.DlT[sp];
+    double *Dv = blk + L.Dv[sp];
+    Deriv4<double> *DW = (Deriv4<double> *)(blk + L.D4[sp]);
     for (int o = lane; o < a; o += 32) {
       Dv[el * a + o] = Dn[o];
-      DgW[(0 * a + o) * n + el] = Dn[a + o];
-      DgW[(1 * a + o) * n + el] = Dn[2 * a + o];
-      DgW[(2 * a + o) * n + el] = Dn[3 * a + o];
-      DlW[o * n + el] = Dn[4 * a + o];
+      DW[o * n + el] = {Dn[a + o], Dn[2 * a + o], Dn[3 * a + o], Dn[4 * a + o]};
     }
     for (int t = lane; t < 3 * N; t += 32) {
       blk[L.gradD + t] = gD[t];

@@ -43,7 +43,8 @@ __global__ void __launch_bounds__(128) k_full_md(DevSys S, Layout L, RunCfg cfg,
   for (int sp = 0; sp < 2; sp++) {
     const int n = sp ? S.nb : S.na, a = S.nact[sp], base = sp ? S.na : 0;
     if (n == 0) continue;
-    double *Dv = blk + L.Dv[sp], *DgT = blk + L.DgT[sp], *DlT = blk + L.DlT[sp];
+    double *Dv = blk + L.Dv[sp];
+    Deriv4<double> *D4 = (Deriv4<double> *)(blk + L.D4[sp]);
     if (do_basis) {
       for (int e = 0; e < n; e++) {
         const double r[3] = {Rs[3 * (base + e)], Rs[3 * (base + e) + 1], Rs[3 * (base + e) + 2]};
@@ -57,10 +58,7 @@ __global__ void __launch_bounds__(128) k_full_md(DevSys S, Layout L, RunCfg cfg,
         }
         for (int o = lane; o < a; o += 32) {
           Dv[e * a + o] = Dn[o];
-          DgT[(0 * a + o) * n + e] = Dn[a + o];
-          DgT[(1 * a + o) * n + e] = Dn[2 * a + o];
-          DgT[(2 * a + o) * n + e] = Dn[3 * a + o];
-          DlT[o * n + e] = Dn[4 * a + o];
+          D4[o * n + e] = {Dn[a + o], Dn[2 * a + o], Dn[3 * a + o], Dn[4 * a + o]};
         }
         __syncwarp();
       }
@@ -102,10 +100,11 @@ __global__ void __launch_bounds__(128) k_full_md(DevSys S, Layout L, RunCfg cfg,
         for (int o = 0; o < n; o++) {
           const int orb = occ[o];
           const double iv = X[o * n + e];
-          lp += DlT[orb * n + e] * iv;
-          gx += DgT[(0 * a + orb) * n + e] * iv;
-          gy += DgT[(1 * a + orb) * n + e] * iv;
-          gz += DgT[(2 * a + orb) * n + e] * iv;
+          const Deriv4<double> v = D4[orb * n + e];
+          lp += v.l * iv;
+          gx += v.x * iv;
+          gy += v.y * iv;
+          gz += v.z * iv;
         }
         double *g = mb[sp].g + ((size_t)c * n + e) * 3;
         g[0] = gx;

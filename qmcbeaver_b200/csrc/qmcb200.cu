@@ -1295,8 +1295,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   for (int sp = 0; sp < 2; sp++) {
     int n = sp ? nb : na, a = nact[sp];
     L.Dv[sp] = take(n * a);
-    L.DgT[sp] = take(3 * a * n);
-    L.DlT[sp] = take(a * n);
+    L.D4[sp] = take(3 * a * n);  // (the block's size predates the interleaved elements: 3 + 1 per pair, padded apart)
+    take(a * n);
     if (md) {
       // two copies of [inverses | grad ratios | (ln|det|, sign, lap, singular)]
       L.mdsz[sp] = (S.ndet * n * n + S.ndet * 3 * n + S.ndet * 4 + 3) & ~3;

@@ -185,10 +185,8 @@ __global__ void __launch_bounds__(32 * kR64MTiles *NH, NH == 2 ? 1 : 2)
           const int el = e - base;
           if (q == 0)
             blk[L.Dv[sp] + el * n + o] = v;
-          else if (q < 4)
-            blk[L.DgT[sp] + ((q - 1) * n + o) * n + el] = v;
           else
-            blk[L.DlT[sp] + o * n + el] = v;
+            blk[L.D4[sp] + 4 * (o * n + el) + q - 1] = v;
         } else {
           rows[((size_t)(w0 + w) * 5 + q) * n + o] = v;
         }

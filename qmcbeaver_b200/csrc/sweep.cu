@@ -24,11 +24,12 @@
 // with one CTA per SM -- proposals 1, basis 7.5, products 6, pair terms 3,
 // Sherman-Morrison 2, ratio sums 7, drift 4.5, acceptance and write back 6 --
 // at 8 warps), which a second CTA on the SM overlaps (16 walkers a CTA: 98 us
-// a step at 16,384 walkers; 32 walkers in one CTA of 16 warps: 126).  128
+// a step at 16,384 walkers; 32 walkers in one CTA of 16 warps: 129; both with
+// the derivative rows as four matrices).  128
 // registers a thread; with 223 KB of shared memory the L1 is small, so spilled
 // registers cost L2 latencies and the column of the inverse leaves the
 // registers for the ratio sums.  30 electrons, 15,710 walkers: 225 us a step
-// by the move kernel, 94 here; 10 electrons, 100 walkers: 18 and 10.
+// by the move kernel, 84 here; 10 electrons, 100 walkers: 18 and 9.
 #include "rows64_device.cuh"
 #include "sweep.h"
 
@@ -260,33 +261,23 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   //      spin's orbitals are clamped and their terms dropped.
   double lp = 0.0, gn[3] = {0.0, 0.0, 0.0};
   {
-    const double *Dg = blk + L.DgT[sp] + cc;
-    const double *Dl = blk + L.DlT[sp] + cc;
+    const Deriv4<double> *D4 = (const Deriv4<double> *)(blk + L.D4[sp]) + cc;
     const bool own = c == el;
     constexpr int kB = 8;
 #pragma unroll 1
     for (int o0 = 0; o0 < n; o0 += kB) {
-      double g[4][kB];
+      Deriv4<double> g[kB];
 #pragma unroll
-      for (int u = 0; u < kB; u++) {
-        const int o = min(o0 + u, n - 1);
-#pragma unroll
-        for (int k = 0; k < 3; k++) g[k][u] = __ldcg(Dg + (k * n + o) * n);
-        g[3][u] = __ldcg(Dl + o * n);
-      }
+      for (int u = 0; u < kB; u++) g[u] = ld_deriv<false>(D4 + min(o0 + u, n - 1) * n);
 #pragma unroll
       for (int u = 0; u < kB; u++) {
         const int o = min(o0 + u, n - 1);
         const double iv = o0 + u < n ? sInv[o * n + cc] : 0.0;
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          const double x = D[(k + 1) * Sh::kLdR + o];
-          const double y = own ? x : g[k][u];
-          if (k < 3)
-            gn[k] = fma(y, iv, gn[k]);
-          else
-            lp = fma(y, iv, lp);
-        }
+        const double *Do = D + o;
+        gn[0] = fma(own ? Do[Sh::kLdR] : g[u].x, iv, gn[0]);
+        gn[1] = fma(own ? Do[2 * Sh::kLdR] : g[u].y, iv, gn[1]);
+        gn[2] = fma(own ? Do[3 * Sh::kLdR] : g[u].z, iv, gn[2]);
+        lp = fma(own ? Do[4 * Sh::kLdR] : g[u].l, iv, lp);
       }
     }
     lp = mine ? lp : 0.0;
@@ -465,9 +456,8 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
     if (mine) {
       // lane c writes orbital c of the moved electron's new rows
       blk[L.Dv[sp] + el * n + c] = D[c];
-#pragma unroll
-      for (int k = 0; k < 3; k++) blk[L.DgT[sp] + (k * n + c) * n + el] = D[(k + 1) * Sh::kLdR + c];
-      blk[L.DlT[sp] + c * n + el] = D[4 * Sh::kLdR + c];
+      ((Deriv4<double> *)(blk + L.D4[sp]))[c * n + el] = {D[Sh::kLdR + c], D[2 * Sh::kLdR + c], D[3 * Sh::kLdR + c],
+                                                        D[4 * Sh::kLdR + c]};
     }
 #pragma unroll
     for (int s = 0; s < 2; s++)
