@@ -11,9 +11,9 @@ ROOT = os.path.dirname(PKG)
 CSRC = os.path.join(PKG, "csrc")
 LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libqmcb200.so")
-SOURCES = ["qmcb200.cu", "sweep.cu", "move.cu", "group.cu", "md.cu", "full.cu", "rows64.cu", "cusp_fit.c"]
+SOURCES = ["qmcb200.cu", "sweep.cu", "invert.cu", "move.cu", "group.cu", "md.cu", "full.cu", "rows64.cu", "cusp_fit.c"]
 HEADERS = ["device_common.cuh", "kernels.cuh", "kernels_population.cuh", "population.cuh", "kernels_md.cuh",
-           "kernels_rows.cuh", "rows64_device.cuh", "group.h", "launches.h", "rows64.h", "sweep.h", "cusp_fit.h"]
+           "kernels_rows.cuh", "rows64_device.cuh", "group.h", "launches.h", "rows64.h", "sweep.h", "invert.h", "cusp_fit.h"]
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = [*ARCH_FLAGS, "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
 

@@ -4,10 +4,17 @@
 
 namespace qmcb {
 
-const void *full_fn(bool mixed, bool extras)
+template <bool kRest>
+static const void *full_fn_of(bool mixed, bool extras)
 {
-  if (mixed) return extras ? (const void *)k_full<float, MIXED_TI, true> : (const void *)k_full<float, MIXED_TI, false>;
-  return extras ? (const void *)k_full<double, double, true> : (const void *)k_full<double, double, false>;
+  if (mixed)
+    return extras ? (const void *)k_full<float, MIXED_TI, true, kRest> : (const void *)k_full<float, MIXED_TI, false, kRest>;
+  return extras ? (const void *)k_full<double, double, true, kRest> : (const void *)k_full<double, double, false, kRest>;
+}
+
+const void *full_fn(bool mixed, bool extras, bool rest)
+{
+  return rest ? full_fn_of<true>(mixed, extras) : full_fn_of<false>(mixed, extras);
 }
 
 }  // namespace qmcb

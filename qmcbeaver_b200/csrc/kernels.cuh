@@ -84,6 +84,8 @@ __host__ __device__ inline int full_scratch_doubles(int N, int K, int nmax)
 {
   return even(5 * (K + 1) + 5 * nmax + nmax * nmax + 3 * nmax + 3 * N + kPart + 8);
 }
+// k_full after the rows and inverses are stored: the positions.
+__host__ __device__ inline int rest_scratch_doubles(int N) { return even(3 * N); }
 // The refresh of stored Slater values (k_full with do_basis = 0) needs no
 // basis rows and no new-row space: a smaller per-warp scratch, more warps per SM.
 __host__ __device__ inline int refresh_scratch_doubles(int N, int nmax)
@@ -460,13 +462,16 @@ __device__ inline double psi_lap_warp(int N, const double *gD, const double *Ux,
 }
 
 // ------------------------------------------------------------------------
-// Full evaluation (do_basis = true: QMCSCFJastrow::evaluate with whichE = -1)
-// or refresh from the stored Slater values (do_basis = false).
+// Full evaluation (do_basis = 1: QMCSCFJastrow::evaluate with whichE = -1),
+// refresh from the stored Slater values (0), or the part of either that
+// follows the stored rows and inverses (2: rows64.cu, invert.cu ran before).
 // R_in: [num][N][3] positions to store first (null: use the stored ones).
-template <typename TS, typename TI, bool kExtras>
-__global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, double *state, const int *slots,
-                                              int num, const int *d_num, const double *R_in, int do_basis,
-                                              EvalOut out)
+// kRest: do_basis is 2, and nothing else is compiled in.
+template <typename TS, typename TI, bool kExtras, bool kRest>
+__global__ void __launch_bounds__(128, kRest && !kExtras ? 5 : 1)
+    k_full(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
+           double *state, const int *slots, int num, const int *d_num, const double *R_in, int do_basis,
+           const __grid_constant__ EvalOut out)
 {
   extern __shared__ double smem[];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -476,7 +481,9 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
   const int N = S.N, K = S.K, nmax = max(S.na, S.nb);
   const int slot = slots ? slots[wi] : wi;
   double *blk = state + (size_t)slot * L.stride;
-  double *sm = smem + (size_t)warp * (do_basis ? full_scratch_doubles(N, K, nmax) : refresh_scratch_doubles(N, nmax));
+  double *sm = smem + (size_t)warp * (kRest      ? rest_scratch_doubles(N)
+                                      : do_basis ? full_scratch_doubles(N, K, nmax)
+                                                 : refresh_scratch_doubles(N, nmax));
   const int ldc = K + 1;
   double *chi = sm;
   double *Dn = chi + 5 * ldc;
@@ -485,7 +492,7 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
   double *vv = A + nmax * nmax;
   double *piv = vv + nmax;
   double *col = piv + nmax;
-  double *Rs = col + nmax;
+  double *Rs = kRest ? sm : col + nmax;
   double *R = blk + L.R;
   double *sc = blk + L.sc;
 
@@ -508,7 +515,7 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
     // sums here always run in FP64 (this is the refresh of the mixed path)
     TS *Dv = (TS *)(blk + L.Dv[sp]);
     Deriv4<TS> *D4 = (Deriv4<TS> *)(blk + L.D4[sp]);
-    if (do_basis) {
+    if (!kRest && do_basis) {
       for (int e = 0; e < n; e++) {
         double r[3] = {Rs[3 * (base + e)], Rs[3 * (base + e) + 1], Rs[3 * (base + e) + 2]};
         basis_shells_warp(S, r, chi, ldc);
@@ -526,19 +533,24 @@ __global__ void __launch_bounds__(128) k_full(DevSys S, Layout L, RunCfg cfg, do
         __syncwarp();
       }
     }
-    for (int t = lane; t < n * n; t += 32) A[t] = (double)Dv[t];
-    __syncwarp();
-    double logdet, sign;
-    bool ok = gj_inverse_warp(A, vv, piv, col, n, logdet, sign);
-    if (!ok) bad = true;
     TI *Inv = (TI *)(blk + L.Inv[sp]);
-    for (int t = lane; t < n * n; t += 32) Inv[t] = (TI)X[t];
+    double logdet = sc[SC_LOGDET_A + sp], sign = sc[SC_SIGN_A + sp];
+    if (kRest) {
+      if (sign == 0.0) bad = true;
+    } else {
+      for (int t = lane; t < n * n; t += 32) A[t] = (double)Dv[t];
+      __syncwarp();
+      bool ok = gj_inverse_warp(A, vv, piv, col, n, logdet, sign);
+      if (!ok) bad = true;
+      for (int t = lane; t < n * n; t += 32) Inv[t] = (TI)X[t];
+    }
     // ratio sums (QMcBeaver/src/QMCSlater.cpp:741-762)
     double lp = 0.0;
     for (int e = lane; e < n; e += 32) {
       double gx = 0, gy = 0, gz = 0;
+#pragma unroll 4
       for (int o = 0; o < n; o++) {
-        double iv = X[o * n + e];
+        double iv = kRest ? (double)Inv[o * n + e] : X[o * n + e];
         const Deriv4<TS> g = ld_deriv<true>(&D4[o * n + e]);
         lp += (double)g.l * iv;
         gx += (double)g.x * iv;

@@ -16,8 +16,8 @@ struct GroupMember;
 
 // k_move<metropolis, float or double, ..., extras, ginv> (move.cu)
 const void *move_fn(bool metropolis, bool mixed, bool extras, bool ginv);
-// k_full<float or double, ..., extras> (full.cu)
-const void *full_fn(bool mixed, bool extras);
+// k_full<float or double, ..., extras, rest> (full.cu)
+const void *full_fn(bool mixed, bool extras, bool rest);
 // k_full_md, k_move_md<metropolis> (md.cu)
 const void *full_md_fn();
 const void *move_md_fn(bool metropolis);

@@ -24,6 +24,7 @@
 #include "kernels.cuh"
 #include "kernels_md.cuh"
 #include "kernels_rows.cuh"
+#include "invert.h"
 #include "launches.h"
 #include "population.cuh"
 #include "rows64.h"
@@ -1393,8 +1394,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   // (each launching with its own size) never undercut one another
   for (int k = 0; k < 16; k++)
     CKC(cudaFuncSetAttribute(move_fn(k & 1, k & 2, k & 4, k & 8), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  for (int k = 0; k < 4; k++)
-    CKC(cudaFuncSetAttribute(full_fn(k & 1, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
+  for (int k = 0; k < 8; k++)
+    CKC(cudaFuncSetAttribute(full_fn(k & 1, k & 2, k & 4), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
   for (const void *fn : {full_md_fn(), move_md_fn(true), move_md_fn(false)})
     CKC(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
   // Below one full wave of the fused move kernel (a warp per walker, its
@@ -1533,23 +1534,30 @@ static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
                         const int *d_num, const double *R_in, int do_basis, EvalOut o)
 {
   // list entries [0, num) (d_num: device count), grid sized for `cap`;
-  // the refresh (do_basis = 0) runs with its smaller per-warp scratch
+  // the refresh (do_basis = 0, 2) runs with its smaller per-warp scratch
   if (do_basis && h->params.precision != QMCB_PREC_MIXED && h->r64.nchunk > 0 && !h->sys.cusp &&
       (h->N > 4 || cap >= 1024)) {
     // all electrons' orbital rows into the walker state, then the refresh of
     // the stored rows (with the caller's positions): 1 / 4,096 walkers, us,
-    // one warp a walker and this way: 3 electrons 24, 71 and 26, 57; 10: 79,
-    // 254 and 42, 116; 30: 301, 1,262 and 96, 455; 100: 5,083, 38,592 and 564,
-    // 7,718.  (The cusp replacement works on rows before they are stored.)
+    // one warp a walker and this way: 3 electrons 24, 71 and 25, 41; 10: 79,
+    // 254 and 37, 84; 30: 301, 1,262 and 66, 331; 100: 5,083, 38,592 and 357,
+    // 6,673.  (The cusp replacement works on rows before they are stored.)
     for (int sp = 0; sp < 2; sp++)
       rows64_launch(R64_ALL, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num, R_in, MoveArgs{}, sp,
                     nullptr);
     do_basis = 0;
   }
-  const int wpb = do_basis ? h->wpb_full : h->wpb_refresh;
+  if (!do_basis && h->nmax <= kInvertMax) {
+    // the inverses in a kernel of their own (invert.cu), then the rest
+    invert_launch(h->params.precision == QMCB_PREC_MIXED, h->sys, h->lay, h->d_state, cap, st, slots, num, d_num);
+    do_basis = 2;
+  }
+  const int wpb = do_basis == 2 ? kMaxWarpsPerBlock : do_basis ? h->wpb_full : h->wpb_refresh;
   const dim3 g((cap + wpb - 1) / wpb), b(32 * wpb);
-  const size_t sm = do_basis ? h->smem_full : h->smem_refresh;
-  launch_kernel(full_fn(h->params.precision == QMCB_PREC_MIXED, h->extras), g, b, sm, st, h->sys, h->lay, cfg,
+  const size_t sm = do_basis == 2 ? sizeof(double) * (size_t)rest_scratch_doubles(h->N) * wpb
+                    : do_basis    ? h->smem_full
+                                  : h->smem_refresh;
+  launch_kernel(full_fn(h->params.precision == QMCB_PREC_MIXED, h->extras, do_basis == 2), g, b, sm, st, h->sys, h->lay, cfg,
                 h->d_state, slots, num, d_num, R_in, do_basis, o);
 }
 
