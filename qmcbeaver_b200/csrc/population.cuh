@@ -26,21 +26,21 @@ __global__ void k_energy(EnergyCtl *ectl, const double *stats, int min_samples_o
   update_energy(ectl, stats, min_samples_ok, dyn_dt, dt);
 }
 
-// Packs R, weight, E_L, log|psi|, sign of the first n live walkers into
-// out[n][3N + 4] for one device-to-host copy.
+// R [n][3N], then weight, E_L, log|psi|, sign [n] each of the first n live
+// walkers into out.
 __global__ void k_gather(const double *state, Layout L, int N, const int *live, int n, double *out)
 {
   const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = lane_id();
   if (w >= n) return;
   const double *blk = state + (size_t)live[w] * L.stride;
-  double *o = out + (size_t)w * (3 * N + 4);
+  double *o = out + (size_t)w * 3 * N, *s = out + (size_t)n * 3 * N + w;
   for (int t = lane; t < 3 * N; t += 32) o[t] = blk[L.R + t];
   if (lane == 0) {
     const double *sc = blk + L.sc;
-    o[3 * N] = sc[SC_WEIGHT];
-    o[3 * N + 1] = sc[SC_EL];
-    o[3 * N + 2] = sc[SC_LOGDET_A] + sc[SC_LOGDET_B] + sc[SC_U];
-    o[3 * N + 3] = sc[SC_SIGN_A] * sc[SC_SIGN_B];
+    s[0] = sc[SC_WEIGHT];
+    s[(size_t)n] = sc[SC_EL];
+    s[2 * (size_t)n] = sc[SC_LOGDET_A] + sc[SC_LOGDET_B] + sc[SC_U];
+    s[3 * (size_t)n] = sc[SC_SIGN_A] * sc[SC_SIGN_B];
   }
 }
 

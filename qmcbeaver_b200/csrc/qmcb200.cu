@@ -35,6 +35,10 @@ using namespace qmcb;
 namespace {
 
 const int kMaxWarpsPerBlock = 4;
+// Evaluate calls whose inputs and outputs fit these go through pinned staging:
+// one copy each way by the DMA engine instead of a pageable copy per array
+// (one walker of water: 137 us a call with eight copies back, 70 so).
+const size_t kStageBytes = 65536;
 const int kStagedInverseMax = 16;  // largest spin whose inverse the move kernel stages in shared memory
 
 std::string g_create_error;
@@ -122,6 +126,10 @@ struct qmcb_handle {
   cudaEvent_t done_ev[2] = {nullptr, nullptr};
   int n_flight = 0;           // batches enqueued and not yet collected
   EnergyCtl *h_ectl = nullptr;  // pinned [4]: E_T / E_est uploads of qmcb_set_params
+  // pinned staging of small evaluate calls (kStageBytes each way; every call
+  // that uses it waits for its copies before it returns)
+  unsigned char *h_stage_in = nullptr, *h_stage_out = nullptr;
+  void *h_pinned = nullptr;     // the one allocation behind all of these
   cudaEvent_t ectl_ev[4] = {nullptr, nullptr, nullptr, nullptr};  // each slot's copy done
   int ectl_next = 0;
   int head = 0;               // slot of the oldest of them
@@ -1359,9 +1367,17 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   CKC(cudaMalloc(&h->d_R, sizeof(double) * (size_t)max_walkers * 3 * h->N));
   CKC(cudaMalloc(&h->d_out, sizeof(double) * (size_t)max_walkers * (6 * h->N + 8)));
   CKC(cudaMalloc(&h->d_status, max_walkers));
-  CKC(cudaMallocHost(&h->h_stats, sizeof(double) * 2 * ST_COUNT));
-  CKC(cudaMallocHost(&h->h_ctl, sizeof(int) * 2 * 4));
-  CKC(cudaMallocHost(&h->h_ectl, sizeof(EnergyCtl) * 4));
+  {
+    const size_t stats = (sizeof(double) * 2 * ST_COUNT + 255) & ~(size_t)255;
+    CKC(cudaMallocHost(&h->h_pinned, stats + 512 + 2 * kStageBytes));
+    unsigned char *p = (unsigned char *)h->h_pinned;
+    h->h_stats = (double *)p;
+    h->h_ctl = (int *)(p + stats);
+    static_assert(sizeof(EnergyCtl) * 4 <= 256, "the pinned block's control part");
+    h->h_ectl = (EnergyCtl *)(p + stats + 256);
+    h->h_stage_in = p + stats + 512;
+    h->h_stage_out = h->h_stage_in + kStageBytes;
+  }
   for (int k = 0; k < 4; k++) CKC(cudaEventCreateWithFlags(&h->ectl_ev[k], cudaEventDisableTiming));
   CKC(cudaEventCreateWithFlags(&h->done_ev[0], cudaEventDisableTiming));
   CKC(cudaEventCreateWithFlags(&h->done_ev[1], cudaEventDisableTiming));
@@ -1445,9 +1461,7 @@ int qmcb_destroy(qmcb_handle *h)
     if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : h->ectl_ev)
     if (e) cudaEventDestroy(e);
-  if (h->h_ectl) cudaFreeHost(h->h_ectl);
-  if (h->h_stats) cudaFreeHost(h->h_stats);
-  if (h->h_ctl) cudaFreeHost(h->h_ctl);
+  if (h->h_pinned) cudaFreeHost(h->h_pinned);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
   return QMCB_OK;
@@ -1606,6 +1620,8 @@ struct EvalDst {
   void *host[8], *dev[8], *kernel[8];
   size_t bytes[8];
   bool mapped[8];
+  bool staged;         // small, nothing mapped: the whole device buffer by one copy into the pinned staging
+  size_t total;        // its bytes
 };
 
 static EvalOut eval_destinations(qmcb_handle *h, bool direct, int num, unsigned mask, double *log_abs_psi, double *sign,
@@ -1622,6 +1638,12 @@ static EvalOut eval_destinations(qmcb_handle *h, bool direct, int num, unsigned 
   const size_t bytes[8] = {sizeof(double) * num, sizeof(double) * num, sizeof(double) * 3 * N * num,
                            sizeof(double) * 3 * N * num, sizeof(double) * num, sizeof(double) * num,
                            sizeof(double) * 3 * num, (size_t)num};
+  // (the status bytes follow the doubles: the buffer has 6 N + 8 per walker)
+  d.total = sizeof(double) * (6 * N + 7) * num + num;
+  d.staged = d.total <= kStageBytes;
+  for (int i = 0; i < 8 && d.staged; i++)
+    if ((mask & bit[i]) && host[i] && mapped_device_ptr(host[i])) d.staged = false;
+  if (d.staged) dev[7] = o_mg + 3 * N * num;
   for (int i = 0; i < 8; i++) {
     d.host[i] = host[i];
     d.dev[i] = dev[i];
@@ -1641,8 +1663,9 @@ static EvalOut eval_destinations(qmcb_handle *h, bool direct, int num, unsigned 
 
 // After the kernel (enqueued on st): the mapped per-walker outputs by one
 // k_put_outputs launch, the pageable ones by one copy each.
-static cudaError_t eval_deliver(const EvalDst &d, cudaStream_t st)
+static cudaError_t eval_deliver(qmcb_handle *h, const EvalDst &d, cudaStream_t st)
 {
+  if (d.staged) return cudaMemcpyAsync(h->h_stage_out, h->d_out, d.total, cudaMemcpyDeviceToHost, st);
   PutList P{};
   int nput = 0;
   size_t most = 0;
@@ -1665,6 +1688,30 @@ static cudaError_t eval_deliver(const EvalDst &d, cudaStream_t st)
     return cudaGetLastError();
   }
   return cudaSuccess;
+}
+
+// The staged outputs into the caller's arrays, once the stream is idle.
+static void eval_unpack(qmcb_handle *h, const EvalDst &d)
+{
+  if (!d.staged) return;
+  for (int i = 0; i < 8; i++)
+    if (d.kernel[i])
+      std::memcpy(d.host[i], h->h_stage_out + ((unsigned char *)d.dev[i] - (unsigned char *)h->d_out), d.bytes[i]);
+}
+
+// Slots and positions of an evaluate call to the device (through the pinned
+// staging when they fit).
+static cudaError_t eval_upload(qmcb_handle *h, const int *slots, int num, const double *R, size_t doubles,
+                               cudaStream_t st)
+{
+  const size_t nr = sizeof(double) * doubles, ns = sizeof(int) * num;
+  const void *r = R, *s = slots;
+  if (nr + ns <= kStageBytes) {
+    r = std::memcpy(h->h_stage_in, R, nr);
+    s = std::memcpy(h->h_stage_in + nr, slots, ns);
+  }
+  const cudaError_t e = cudaMemcpyAsync(h->d_slots, s, ns, cudaMemcpyHostToDevice, st);
+  return e != cudaSuccess ? e : cudaMemcpyAsync(h->d_R, r, nr, cudaMemcpyHostToDevice, st);
 }
 
 static int launch_eval(qmcb_handle *h, int which_e, const int *d_slots, int num, const double *d_R, EvalOut o,
@@ -1731,8 +1778,7 @@ int qmcb_evaluate(qmcb_handle *h, int which_e, const int *slots, int num, const 
   if (num == 0) return QMCB_OK;
   const int N = h->N;
   cudaStream_t st = h->stream;
-  CK(cudaMemcpyAsync(h->d_slots, slots, sizeof(int) * num, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_R, R, sizeof(double) * (size_t)num * 3 * N, cudaMemcpyHostToDevice, st));
+  CK(eval_upload(h, slots, num, R, (size_t)num * 3 * N, st));
   // every non-NULL output is returned
   EvalDst dst;
   const EvalOut o = eval_destinations(h, which_e < 0 || !sweep_moves(h), num, QMCB_OUT_ALL, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
@@ -1740,11 +1786,12 @@ int qmcb_evaluate(qmcb_handle *h, int which_e, const int *slots, int num, const 
   int rc = launch_eval(h, which_e, h->d_slots, num, h->d_R, o, st);
   if (rc) return rc;
   if (which_e < 0) h->evaluated_once = true;
-  CK(eval_deliver(dst, st));
+  CK(eval_deliver(h, dst, st));
   int rows_err = 0;
   if (rows_mode(h->params.precision) && which_e >= 0)
     CK(cudaMemcpyAsync(&rows_err, h->d_ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  eval_unpack(h, dst);
   if (rows_err) return fail(h, QMCB_E_CUDA, "qmcb_evaluate: the tensor-core contraction gave up waiting (rows not written)");
   return QMCB_OK;
 }
@@ -1767,18 +1814,18 @@ int qmcb_evaluate_moved(qmcb_handle *h, int which_e, const int *slots, int num, 
     return fail(h, QMCB_E_ARG, "qmcb_evaluate_moved: an output selected in out_mask is NULL");
   if (num == 0) return QMCB_OK;
   cudaStream_t st = h->stream;
-  CK(cudaMemcpyAsync(h->d_slots, slots, sizeof(int) * num, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_R, r_moved, sizeof(double) * 3 * (size_t)num, cudaMemcpyHostToDevice, st));
+  CK(eval_upload(h, slots, num, r_moved, 3 * (size_t)num, st));
   EvalDst dst;
   const EvalOut o = eval_destinations(h, !sweep_moves(h), num, out_mask, log_abs_psi, sign, grad, mod_grad, lap, e_local, pe,
                                       status, dst);
   int rc = launch_eval(h, which_e, h->d_slots, num, h->d_R, o, st, 1);
   if (rc) return rc;
-  CK(eval_deliver(dst, st));
+  CK(eval_deliver(h, dst, st));
   int rows_err = 0;
   if (rows_mode(h->params.precision))
     CK(cudaMemcpyAsync(&rows_err, h->d_ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  eval_unpack(h, dst);
   if (rows_err) return fail(h, QMCB_E_CUDA, "qmcb_evaluate_moved: the tensor-core contraction gave up waiting");
   return QMCB_OK;
 }
@@ -2044,20 +2091,28 @@ int qmcb_get_walkers(qmcb_handle *h, int n, double *R, double *weight, double *e
   if (n < 0 || n > h->n_live_host) return fail(h, QMCB_E_ARG, "qmcb_get_walkers: n beyond live walkers");
   if (n == 0) return QMCB_OK;
   cudaStream_t st = h->stream;
-  const int N = h->N, rec = 3 * N + 4;
-  k_gather<<<(n + 3) / 4, 128, 0, st>>>(h->d_state, h->lay, N, h->d_live, n, h->d_out);
+  // the arrays one after another on the device, then straight into the
+  // caller's (few small ones: by one copy through a buffer)
+  const size_t count[5] = {(size_t)n * 3 * h->N, (size_t)n, (size_t)n, (size_t)n, (size_t)n};
+  double *host[5] = {R, weight, e_local, log_abs_psi, sign};
+  k_gather<<<(n + 3) / 4, 128, 0, st>>>(h->d_state, h->lay, h->N, h->d_live, n, h->d_out);
   CK(cudaGetLastError());
-  std::vector<double> buf((size_t)n * rec);
-  CK(cudaMemcpyAsync(buf.data(), h->d_out, sizeof(double) * buf.size(), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  for (int i = 0; i < n; i++) {
-    const double *o = buf.data() + (size_t)i * rec;
-    if (R) std::memcpy(R + (size_t)i * 3 * N, o, sizeof(double) * 3 * N);
-    if (weight) weight[i] = o[3 * N];
-    if (e_local) e_local[i] = o[3 * N + 1];
-    if (log_abs_psi) log_abs_psi[i] = o[3 * N + 2];
-    if (sign) sign[i] = o[3 * N + 3];
+  const size_t total = count[0] + 4 * (size_t)n;
+  std::vector<double> buf;
+  if (sizeof(double) * total <= 4 * kStageBytes) {
+    buf.resize(total);
+    CK(cudaMemcpyAsync(buf.data(), h->d_out, sizeof(double) * total, cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
   }
+  size_t at = 0;
+  for (int k = 0; k < 5; at += count[k++]) {
+    if (!host[k]) continue;
+    if (!buf.empty())
+      std::memcpy(host[k], buf.data() + at, sizeof(double) * count[k]);
+    else
+      CK(cudaMemcpyAsync(host[k], h->d_out + at, sizeof(double) * count[k], cudaMemcpyDeviceToHost, st));
+  }
+  CK(cudaStreamSynchronize(st));
   return QMCB_OK;
 }
 
