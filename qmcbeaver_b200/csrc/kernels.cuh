@@ -1543,10 +1543,18 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
   }
 }
 
+// The parameters stay in constant memory (__grid_constant__): passed by value
+// to functions that are not inlined they were copied to every thread's stack,
+// 1,408 bytes with the extras, whose 96-register cap (5 blocks per SM) also
+// spilled; with 3 blocks and no copies a step of 16 electrons with cusps,
+// three-body terms and Umrigar93 moves takes 151 us instead of 200 (4,096
+// walkers), one of 12 determinants 100 instead of 130.
 template <bool kMetropolis, typename TS, typename TI, bool kExtras, bool kGInv>
-__global__ void __launch_bounds__(128, kGInv ? 3 : 5) k_move(DevSys S, Layout L, RunCfg cfg, double *state, const int *slots,
-                                              int num, const int *d_num, const double *R_in, MoveArgs mv,
-                                              const EnergyCtl *ectl, double *stats, EvalOut out)
+__global__ void __launch_bounds__(128, kGInv || kExtras ? 3 : 5)
+    k_move(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
+           double *state, const int *slots, int num, const int *d_num, const double *R_in,
+           const __grid_constant__ MoveArgs mv, const EnergyCtl *ectl, double *stats,
+           const __grid_constant__ EvalOut out)
 {
   extern __shared__ double smem[];
   const int warp = threadIdx.x >> 5;

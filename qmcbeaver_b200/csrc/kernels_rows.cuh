@@ -128,7 +128,8 @@ __host__ __device__ inline int rows_prep_doubles(int N, int K, int nslot)
 }
 
 template <bool kMetropolis, bool kExtras>
-__global__ void __launch_bounds__(128) k_rows_prep(DevSys S, Layout L, RunCfg cfg, const double *state,
+__global__ void __launch_bounds__(128) k_rows_prep(const __grid_constant__ DevSys S, const __grid_constant__ Layout L,
+                                                    const __grid_constant__ RunCfg cfg, const double *state,
                                                     const int *slots, int num, const int *d_num, const double *R_in,
                                                     MoveArgs mv, int ksteps, signed char *A, double *rscale)
 {
@@ -552,7 +553,8 @@ __host__ __device__ inline uint32_t bf16_bits(double v)
 }
 
 template <bool kMetropolis, bool kExtras, int kPlanes>
-__global__ void __launch_bounds__(128) k_rows_prep_bf(DevSys S, Layout L, RunCfg cfg, const double *state,
+__global__ void __launch_bounds__(128) k_rows_prep_bf(const __grid_constant__ DevSys S, const __grid_constant__ Layout L,
+                                                       const __grid_constant__ RunCfg cfg, const double *state,
                                                        const int *slots, int num, const int *d_num,
                                                        const double *R_in, MoveArgs mv, int ksteps,
                                                        unsigned char *A)

@@ -6,9 +6,10 @@ namespace qmcb {
 
 // ------------------------------------------------------------------------
 // Full evaluation (do_basis = true) or refresh from the stored rows.
-__global__ void __launch_bounds__(128) k_full_md(DevSys S, Layout L, RunCfg cfg, double *state, const int *slots,
-                                                 int num, const int *d_num, const double *R_in, int do_basis,
-                                                 EvalOut out)
+__global__ void __launch_bounds__(128)
+    k_full_md(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
+              double *state, const int *slots, int num, const int *d_num, const double *R_in, int do_basis,
+              const __grid_constant__ EvalOut out)
 {
   extern __shared__ double smem[];
   const int lane = lane_id(), warp = threadIdx.x >> 5;
@@ -166,9 +167,11 @@ __global__ void __launch_bounds__(128) k_full_md(DevSys S, Layout L, RunCfg cfg,
 }
 
 template <bool kMetropolis>
-__global__ void __launch_bounds__(128, 3) k_move_md(DevSys S, Layout L, RunCfg cfg, double *state, const int *slots,
-                                                 int num, const int *d_num, const double *R_in, MoveArgs mv,
-                                                 const EnergyCtl *ectl, double *stats, EvalOut out)
+__global__ void __launch_bounds__(128, 3)
+    k_move_md(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
+              double *state, const int *slots, int num, const int *d_num, const double *R_in,
+              const __grid_constant__ MoveArgs mv, const EnergyCtl *ectl, double *stats,
+              const __grid_constant__ EvalOut out)
 {
   extern __shared__ double smem[];
   const int warp = threadIdx.x >> 5;
