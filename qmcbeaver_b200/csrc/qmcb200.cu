@@ -673,7 +673,9 @@ static void launch_move(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
     ps.end(st);
     return;
   }
-  if (rows64_moves(h, cap)) {
+  // (the rows buffer is the handle's: calls for disjoint walkers on callers'
+  // streams may overlap, and evaluate their rows in the move kernel)
+  if (rows64_moves(h, cap) && st == h->stream) {
     {
       ProfScope ps(h, QMCB_KERNEL_ROWS_PREP, st);
       rows64_launch(kMetropolis ? R64_PROPOSE : R64_GIVEN, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num,
@@ -1432,7 +1434,16 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
     CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, move_fn(true, false, h->extras, h->ginv),
                                                       32 * h->wpb_move, h->smem_move));
     h->rows64_from = h->nmax > 64 ? 1 : n_sm * per_sm * h->wpb_move + 1;
-    if (max_walkers >= h->rows64_from) CKC(cudaMalloc(&h->d_rows64, sizeof(double) * (size_t)max_walkers * 5 * h->nmax));
+    if (max_walkers >= h->rows64_from) {
+      const cudaError_t e = cudaMalloc(&h->d_rows64, sizeof(double) * (size_t)max_walkers * 5 * h->nmax);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();  // walkers that just fit: moves by the fused kernel
+        h->d_rows64 = nullptr;
+        h->rows64_from = INT_MAX;
+      } else {
+        CKC(e);
+      }
+    }
   }
   // the memsets above ran on the legacy default stream, which does not order
   // against the handle's non-blocking stream: finish them before any work is

@@ -75,3 +75,50 @@ def test_moves_of_many_walkers_match_oracle(ne, nb, odd):
     s = _molecule(ne, nb, odd)
     W = 3201  # more than 148 SMs hold of any molecule; the last tile holds one walker
     _check(s, W, [0, s.n_alpha - 1, ne - 1, 0], np.array([0, 31, 32, 1777, 3199, 3200]))
+
+
+def test_moves_of_disjoint_walkers_on_two_streams_match_oracle():
+    # evaluate_device on two callers' streams, half of the walkers each: the
+    # calls may overlap, so nothing but the walkers' own state may be written
+    import ctypes
+    import torch
+    from oracle.evaluators import OracleEvaluator
+    s, W, watched = _molecule(130, 265, False), 1024, np.array([0, 511, 512, 1023])
+    orc = OracleEvaluator(s, qf_mod=2, dt=0.01)
+    f = QMCB200Functions(s, W, qf_modification=2, dt=0.01)
+    ws = orc.new_walkers(len(watched))
+    R = s.initial_positions(W, seed=4, sigma=0.7)
+    f.evaluate(np.arange(W), R, -1)
+    orc.evaluate(ws, R[watched], -1)
+    worst = slater_conditions(orc, ws, s)
+    rng = np.random.default_rng(5)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    slots = torch.arange(W, dtype=torch.int32, device="cuda")
+    sides = []
+    for e in (0, 64, 65, 129):
+        R[:, e] += 0.2 * rng.standard_normal((W, 3))
+        out = [torch.zeros(W * k, dtype=torch.float64, device="cuda") for k in (1, 1, 390, 390, 1, 1, 3)]
+        sides.append((e, torch.tensor(R, device="cuda"), out, torch.zeros(W, dtype=torch.uint8, device="cuda")))
+        orc.evaluate(ws, R[watched], e)
+        worst = np.maximum(worst, slater_conditions(orc, ws, s))
+    torch.cuda.synchronize()
+    for e, r, out, status in sides:
+        for half, st in enumerate(streams):
+            at = half * (W // 2)
+            args = [ctypes.c_void_p(x.data_ptr() + at * x.element_size() * (x.numel() // W)) for x in out + [status]]
+            rc = f.lib.qmcb_evaluate_device(f.h, e, ctypes.c_void_p(slots.data_ptr() + 4 * at), W // 2,
+                                            ctypes.c_void_p(r.data_ptr() + 8 * 390 * at), *args,
+                                            ctypes.c_void_p(st.cuda_stream))
+            assert rc == 0
+    torch.cuda.synchronize()
+    ref = orc.results(ws)
+    slope, limit = cond_bounds(s)
+    names = ("log_abs_psi", "sign", "grad", "mod_grad", "lap", "e_local")
+    out = {k: v.cpu().numpy().reshape(W, -1)[watched].reshape(np.shape(ref[k])) for k, v in zip(names, sides[-1][2])}
+    out["potential"] = sides[-1][2][-1].cpu().numpy().reshape(W, 3)[watched, 0]
+    amp = (np.abs(ref["lap"]) / 2 + np.abs(ref["potential"])) / np.maximum(np.abs(ref["e_local"]), 1.0)
+    for i in range(len(watched)):
+        one = np.arange(len(watched)) == i
+        compare(out, ref, max(PARITY_RTOL, slope * worst[i]) if worst[i] >= limit else PARITY_RTOL,
+                f"walker {watched[i]} (cond {worst[i]:.1e})", mask=one, kappa=amp)
+    f.close()
