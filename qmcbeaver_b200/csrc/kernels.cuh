@@ -466,9 +466,13 @@ __device__ inline double psi_lap_warp(int N, const double *gD, const double *Ux,
 // refresh from the stored Slater values (0), or the part of either that
 // follows the stored rows and inverses (2: rows64.cu, invert.cu ran before).
 // R_in: [num][N][3] positions to store first (null: use the stored ones).
-// kRest: do_basis is 2, and nothing else is compiled in.
-template <typename TS, typename TI, bool kExtras, bool kRest>
-__global__ void __launch_bounds__(128, kRest && !kExtras ? 5 : 1)
+// kRest: do_basis is 2, and nothing else is compiled in.  kDense (rest with
+// extras): four blocks per SM, 128 registers, instead of two at 236, for walkers
+// above what two blocks hold (refresh of 1,024 / 4,096 / 8,192 walkers, us, two
+// and four: 16 electrons 109, 347, 648 and 109, 263, 487; 40: 736, 2,625, 4,915
+// and 744, 1,858, 3,573; 512 walkers of 40: 617 and 650).
+template <typename TS, typename TI, bool kExtras, bool kRest, bool kDense>
+__global__ void __launch_bounds__(128, kDense ? 4 : kRest && !kExtras ? 5 : 1)
     k_full(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
            double *state, const int *slots, int num, const int *d_num, const double *R_in, int do_basis,
            const __grid_constant__ EvalOut out)
@@ -1548,9 +1552,11 @@ __device__ __forceinline__ void move_walker(const DevSys &S, const Layout &L, co
 // 1,408 bytes with the extras, whose 96-register cap (5 blocks per SM) also
 // spilled; with 3 blocks and no copies a step of 16 electrons with cusps,
 // three-body terms and Umrigar93 moves takes 151 us instead of 200 (4,096
-// walkers), one of 12 determinants 100 instead of 130.
-template <bool kMetropolis, typename TS, typename TI, bool kExtras, bool kGInv>
-__global__ void __launch_bounds__(128, kGInv || kExtras ? 3 : 5)
+// walkers), one of 12 determinants 100 instead of 130.  kDense (extras of small
+// spins): four blocks at 128 registers and some spills, chosen by
+// move_dense_wins.
+template <bool kMetropolis, typename TS, typename TI, bool kExtras, bool kGInv, bool kDense>
+__global__ void __launch_bounds__(128, kDense ? 4 : kGInv || kExtras ? 3 : 5)
     k_move(const __grid_constant__ DevSys S, const __grid_constant__ Layout L, const __grid_constant__ RunCfg cfg,
            double *state, const int *slots, int num, const int *d_num, const double *R_in,
            const __grid_constant__ MoveArgs mv, const EnergyCtl *ectl, double *stats,

@@ -16,8 +16,10 @@ struct GroupMember;
 
 // k_move<metropolis, float or double, ..., extras, ginv> (move.cu)
 const void *move_fn(bool metropolis, bool mixed, bool extras, bool ginv);
+const void *move_dense_fn(bool metropolis);  // FP64, extras, small spins: four blocks per SM
 // k_full<float or double, ..., extras, rest> (full.cu)
 const void *full_fn(bool mixed, bool extras, bool rest);
+const void *rest_dense_fn(bool mixed);  // extras, rest: four blocks per SM
 // k_full_md, k_move_md<metropolis> (md.cu)
 const void *full_md_fn();
 const void *move_md_fn(bool metropolis);

@@ -8,10 +8,16 @@ template <bool kMetropolis, typename TS, typename TI>
 static const void *move_fn_of(bool extras, bool ginv)
 {
   if (ginv)
-    return extras ? (const void *)k_move<kMetropolis, TS, TI, true, true>
-                  : (const void *)k_move<kMetropolis, TS, TI, false, true>;
-  return extras ? (const void *)k_move<kMetropolis, TS, TI, true, false>
-                : (const void *)k_move<kMetropolis, TS, TI, false, false>;
+    return extras ? (const void *)k_move<kMetropolis, TS, TI, true, true, false>
+                  : (const void *)k_move<kMetropolis, TS, TI, false, true, false>;
+  return extras ? (const void *)k_move<kMetropolis, TS, TI, true, false, false>
+                : (const void *)k_move<kMetropolis, TS, TI, false, false, false>;
+}
+
+const void *move_dense_fn(bool metropolis)
+{
+  return metropolis ? (const void *)k_move<true, double, double, true, false, true>
+                    : (const void *)k_move<false, double, double, true, false, true>;
 }
 
 const void *move_fn(bool metropolis, bool mixed, bool extras, bool ginv)

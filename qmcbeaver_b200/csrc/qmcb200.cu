@@ -114,6 +114,9 @@ struct qmcb_handle {
   double *d_R = nullptr, *d_out = nullptr;
   unsigned char *d_status = nullptr;
   int n_live_host = 0;
+  int n_start = 0;                 // walkers of the last initialisation
+  int move_wave[2][2] = {};        // walkers one wave of the extras move kernel holds: [rows given][dense], 0: no dense form
+  int rest_wave = INT_MAX;         // walkers one wave of the rest of a full evaluation with extras holds
   double target_weight = 0.0;
   size_t smem_move = 0, smem_full = 0, smem_refresh = 0;
   int wpb_move = 1, wpb_full = 1, wpb_refresh = 1;  // warps (walkers) per CTA of k_move / k_full / the refresh
@@ -409,6 +412,20 @@ void *g_noalloc_w_addr[64];
 void *g_noalloc_i_addr[64];
 }  // namespace
 
+// Whether the extras move kernel runs at four blocks per SM for n walkers.  A
+// wave of four takes 1.2 to 1.3 times one of three (4,096 walkers of 6, 16 and 24
+// electrons with cusps, three-body terms and Umrigar93 moves: two waves of
+// 46, 56 and 74 us against three of 40, 47 and 56), so four win where they save
+// more than a quarter of the waves: 94, 112, 148 us against 120, 140, 169 at
+// 4,096 walkers; at 1,024 (one wave both ways) 51, 57, 69 against 50, 57, 66
+// and at 8,192 (four waves for five) drift moves of 24 electrons 229 against 207.
+static bool move_dense_wins(const qmcb_handle *h, bool rows, int n)
+{
+  const int sparse = h->move_wave[rows][0], dense = h->move_wave[rows][1];
+  if (dense <= 0 || sparse <= 0) return false;
+  return 4 * ((n + dense - 1) / dense) < 3 * ((n + sparse - 1) / sparse);
+}
+
 // One launch of the single-determinant move kernel in the walker state's
 // precision, with the cusp / three-body code only when the system has them.
 static void launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extras, const dim3 &g, const dim3 &b,
@@ -417,8 +434,10 @@ static void launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extr
 {
   // with rows from a batched kernel the scratch has no basis rows
   const Layout &L = mv.rows ? h->lay_rows : h->lay;
-  launch_kernel(move_fn(metropolis, mixed, extras, h->ginv), g, b, sm, st, h->sys, L, cfg, h->d_state, slots, num,
-                d_num, R_in, mv, h->d_ectl, h->d_stats, o);
+  // (the walkers of a run change with branching; their first number decides)
+  const bool dense = extras && !mixed && move_dense_wins(h, mv.rows != nullptr, d_num ? h->n_start : num);
+  launch_kernel(dense ? move_dense_fn(metropolis) : move_fn(metropolis, mixed, extras, h->ginv), g, b, sm, st, h->sys, L,
+                cfg, h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
 }
 
 // The chunks of k_rows64 (struct Rows64): shells dealt, largest first, to the
@@ -1414,7 +1433,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
     CKC(cudaFuncSetAttribute(move_fn(k & 1, k & 2, k & 4, k & 8), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
   for (int k = 0; k < 8; k++)
     CKC(cudaFuncSetAttribute(full_fn(k & 1, k & 2, k & 4), cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
-  for (const void *fn : {full_md_fn(), move_md_fn(true), move_md_fn(false)})
+  for (const void *fn : {full_md_fn(), move_md_fn(true), move_md_fn(false), move_dense_fn(true), move_dense_fn(false),
+                         rest_dense_fn(true), rest_dense_fn(false)})
     CKC(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, max_optin));
   // Below one full wave of the fused move kernel (a warp per walker, its
   // scratch limiting the warps per SM) a step takes one walker's latency, and
@@ -1426,6 +1446,23 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   // one warp's contraction is the longer latency at any size (140 and 196
   // electrons, one walker: 137 and 222 us fused, 128 and 200 in two launches;
   // 1,024 walkers: 368 and 769, 216 and 478).
+  if (!md) {
+    int n_sm = 0, per_sm = 0;
+    CKC(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, h->device));
+    for (int rows = 0; rows < 2 && !h->ginv; rows++)
+      for (int dense = 0; dense < 2; dense++) {
+        const int wpb = rows ? h->wpb_rows : h->wpb_move;
+        CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm,
+                                                          dense ? move_dense_fn(true) : move_fn(true, false, true, false),
+                                                          32 * wpb, rows ? h->smem_rows : h->smem_move));
+        h->move_wave[rows][dense] = n_sm * per_sm * wpb;
+      }
+    if (h->extras) {
+      CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, full_fn(false, true, true), 32 * kMaxWarpsPerBlock,
+                                                        sizeof(double) * (size_t)rest_scratch_doubles(h->N) * kMaxWarpsPerBlock));
+      h->rest_wave = n_sm * per_sm * kMaxWarpsPerBlock;
+    }
+  }
   if (h->r64.nchunk > 0) {
     CKC(sweep_limits(max_optin));
     h->sweep = h->nmax <= kSweepMax && !h->extras && !h->ginv && sweep_smem_bytes(h->nmax, h->lay, h->r64) <= max_optin;
@@ -1582,7 +1619,9 @@ static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
   const size_t sm = do_basis == 2 ? sizeof(double) * (size_t)rest_scratch_doubles(h->N) * wpb
                     : do_basis    ? h->smem_full
                                   : h->smem_refresh;
-  launch_kernel(full_fn(h->params.precision == QMCB_PREC_MIXED, h->extras, do_basis == 2), g, b, sm, st, h->sys, h->lay, cfg,
+  const bool mixed = h->params.precision == QMCB_PREC_MIXED;
+  const bool dense = do_basis == 2 && h->extras && (d_num ? h->n_start : num) > h->rest_wave;
+  launch_kernel(dense ? rest_dense_fn(mixed) : full_fn(mixed, h->extras, do_basis == 2), g, b, sm, st, h->sys, h->lay, cfg,
                 h->d_state, slots, num, d_num, R_in, do_basis, o);
 }
 
@@ -1897,7 +1936,7 @@ int qmcb_init_walkers(qmcb_handle *h, int n, const double *R)
   CK(cudaMemcpyAsync(h->d_ectl, &ec, sizeof(ec), cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_COUNT, st));
   CK(cudaStreamSynchronize(st));
-  h->n_live_host = n;
+  h->n_live_host = h->n_start = n;
   return QMCB_OK;
 }
 
