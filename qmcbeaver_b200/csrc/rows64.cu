@@ -71,8 +71,8 @@ __global__ void __launch_bounds__(32 * kR64MTiles *NH, NH == 2 ? 1 : 2)
   const int splits = kMode == R64_ALL ? gridDim.x / n : gridDim.y;
   const int split = kMode == R64_ALL ? blockIdx.x % splits : blockIdx.y;
   const int e = kMode == R64_ALL ? base + blockIdx.x / splits : mv.e;
-  double *chi = sm64;                           // [kR64Chunk][kR64LdA]
-  double *Cs = chi + kR64Chunk * kR64LdA;       // two buffers [kR64Chunk][kLdB]
+  double *chi = sm64;                           // [kR64Lead + kR64Chunk][kR64LdA], the chunk from row T.lead
+  double *Cs = chi + (kR64Lead + kR64Chunk) * kR64LdA;  // two buffers [kR64Chunk][kLdB]
   double *pos = Cs + 2 * kR64Chunk * kLdB;      // [3][32]
   double *recs = pos + 3 * kR64Walkers;         // two buffers of a chunk's shell records
   const int wi = min(w0 + lane, nw - 1);        // the lanes past the list repeat its last walker
@@ -149,13 +149,14 @@ __global__ void __launch_bounds__(32 * kR64MTiles *NH, NH == 2 ? 1 : 2)
         const int i = s0 + ((s0 / kWarps) & 1 ? kWarps - 1 - warp : warp);
         if (i >= ch.x) continue;
         const double head = rec[i];
-        rows64_shell<kR64Walkers>(rec + __double2hiint(head), __double2loint(head), rx, ry, rz, chi + lane);
+        rows64_shell<kR64Walkers, kMode != R64_ALL>(rec + __double2hiint(head), __double2loint(head), rx, ry, rz, chi + lane);
       }
       // padding functions: their coefficients are zero, their values must be finite
-      for (int k = (ch.z & 0xffff) + warp / 5; k < padded; k += kWarps / 5) chi[k * kR64LdA + 32 * (warp % 5) + lane] = 0.0;
+      for (int k = (ch.z & 0xffff) + warp / 5; k < padded; k += kWarps / 5)
+        chi[(T.lead + k) * kR64LdA + 32 * (warp % 5) + lane] = 0.0;
     }
     __syncthreads();
-    const double *ap = chi + t * kR64LdA + 16 * mtile + g;
+    const double *ap = chi + (T.lead + t) * kR64LdA + 16 * mtile + g;
     const double *bp = Cs + (c & 1) * kR64Chunk * kLdB + t * kLdB + 8 * NT * half + g;
     for (int k = 0; k < padded; k += 8) {
       const double a[4] = {ap[k * kR64LdA], ap[k * kR64LdA + 8], ap[(k + 4) * kR64LdA], ap[(k + 4) * kR64LdA + 8]};

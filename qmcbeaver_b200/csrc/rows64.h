@@ -22,6 +22,11 @@ constexpr int kR64TilesMax = 2 * kR64WarpTiles;  // 8-orbital tiles per CTA
 
 constexpr int kR64RecMax = 1536;             // doubles of a chunk's shell records
 
+// Rows before a chunk's first: the part of a shell that the chunk before it
+// holds (a shell cut by a chunk's end is evaluated for both).  The sweep
+// kernel's tables (spins of 9 to 16) need room behind a chunk's end too.
+constexpr int kR64Lead = 5;
+
 constexpr int kR64Any = 3;                   // shell kind: none of the complete s (0), p (1), d (2) shells
 
 // Tables of the kernel.  A chunk holds at most kR64Chunk functions (padded
@@ -34,6 +39,7 @@ constexpr int kR64Any = 3;                   // shell kind: none of the complete
 struct Rows64 {
   int nchunk;
   int rec_max;          // doubles of the longest chunk's records
+  int lead;             // rows before the chunks' first: 0, or kR64Lead where shells are cut
   const int4 *chunk;    // [nchunk + 1] shells, offset in rec, functions | padded functions << 16, first permuted function
   const double *rec;
   const double *ct[2];  // [permuted functions][ldb] coefficients, zero in the padding
@@ -55,7 +61,8 @@ __host__ __device__ inline int rows64_tiles(int n)
 __host__ __device__ inline int rows64_ldb(int n) { return n > 0 ? 8 * rows64_splits(n) * rows64_halves(n) * rows64_tiles(n) : 8; }
 __host__ __device__ inline int rows64_smem_bytes(int nt, int nh, int rec_max)
 {
-  return (int)sizeof(double) * (kR64Chunk * (kR64LdA + 2 * (8 * nt * nh + 4)) + 3 * kR64Walkers + 2 * rec_max);
+  return (int)sizeof(double) *
+         (kR64Lead * kR64LdA + kR64Chunk * (kR64LdA + 2 * (8 * nt * nh + 4)) + 3 * kR64Walkers + 2 * rec_max);
 }
 
 enum Rows64Mode {

@@ -17,18 +17,33 @@ __device__ __forceinline__ void dmma_m16n8k8(double d[4], const double a[4], dou
       : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
 }
 
+// The squared distance of the exponentials, and that of the Laplacian's sums:
+// the one-walker passes round the latter by itself for a moved electron
+// (basis_function_rows: its squares also serve the powers, so its sum is not
+// fused) and share the former in a full evaluation (shell_members).  Spelled
+// out, so that a walker's rows are the same bits whichever kernel makes them.
+__device__ __forceinline__ double rows64_r2(double x, double y, double z)
+{
+  return fma(z, z, fma(x, x, __dmul_rn(y, y)));
+}
+template <bool kMoved>
+__device__ __forceinline__ double rows64_r2x4(double x, double y, double z, double r2)
+{
+  return 4.0 * (kMoved ? __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)) : r2);
+}
+
 // A shell of any other shape (kR64Any): rec = centre, (L, primitives) in the
 // two words of a double, exponents, then for every function its powers and
 // coefficients.  E0 = sum c e, E1 = sum c a e, El = sum c e (4 r^2 a^2 - (4L + 6) a)
 // as in basis_function_rows.
-template <int TW>
+template <int TW, bool kMoved>
 static __device__ __noinline__ void rows64_shell_any(const double *rec, int nmem, double rx, double ry, double rz,
                                                      double *chi)
 {
   const double x = rx - rec[0], y = ry - rec[1], z = rz - rec[2];
-  const double r2 = x * x + y * y + z * z;
+  const double r2 = rows64_r2(x, y, z);
   const int L = __double2loint(rec[3]), np = __double2hiint(rec[3]);
-  const double Lf = 4.0 * L + 6.0, r2x4 = 4.0 * r2;
+  const double Lf = 4.0 * L + 6.0, r2x4 = rows64_r2x4<kMoved>(x, y, z, r2);
   const double *al = rec + 4, *mem = al + np;
   double E0 = 0.0, E1 = 0.0, El = 0.0;
   for (int m = 0; m < nmem; m++, chi += rows64_pitch(TW), mem += np + 1) {
@@ -62,10 +77,11 @@ static __device__ __noinline__ void rows64_shell_any(const double *rec, int nmem
 }
 
 // One function of a fast shell: its radial sums from the three primitives'
-// e, a e and e a (4 r^2 a - (4L + 6)) and its coefficients, then its five
-// values from its polynomial P, that polynomial's gradient and Laplacian.
+// exponentials e, exponents a and a (4 r^2 a - (4L + 6)) and its coefficients,
+// then its five values from its polynomial P, that polynomial's gradient and
+// Laplacian.  Every operation rounds as in basis_function_rows.
 struct Rows64Radial {
-  double x, y, z, e0[3], e1[3], el[3];
+  double x, y, z, e[3], a[3], l[3];
 };
 template <int TW>
 __device__ __forceinline__ void rows64_function(double *chi, const double *coef, const Rows64Radial &R, double P,
@@ -74,17 +90,19 @@ __device__ __forceinline__ void rows64_function(double *chi, const double *coef,
   double E0 = 0.0, E1 = 0.0, El = 0.0;
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const double c = coef[i];
-    E0 = fma(c, R.e0[i], E0);
-    E1 = fma(c, R.e1[i], E1);
-    El = fma(c, R.el[i], El);
+    const double t = coef[i] * R.e[i];
+    E0 += t;
+    E1 = fma(t, R.a[i], E1);
+    El = fma(t, R.l[i], El);
   }
   const double w = -2.0 * P * E1;
   chi[0] = E0 * P;
-  chi[TW] = fma(E0, Px, R.x * w);
-  chi[2 * TW] = fma(E0, Py, R.y * w);
-  chi[3 * TW] = fma(E0, Pz, R.z * w);
-  chi[4 * TW] = fma(E0, Pl, P * El);
+  // (products rounded before the sum also where a constant polynomial
+  // derivative would let them be fused)
+  chi[TW] = fma(E0, Px, __dmul_rn(R.x, w));
+  chi[2 * TW] = fma(E0, Py, __dmul_rn(R.y, w));
+  chi[3 * TW] = fma(E0, Pz, __dmul_rn(R.z, w));
+  chi[4 * TW] = fma(E0, Pl, __dmul_rn(P, El));
 }
 
 // One shell for this lane's position into the chunk (TW walkers a tile: row =
@@ -93,28 +111,27 @@ __device__ __forceinline__ void rows64_function(double *chi, const double *coef,
 // without a branch or a table lookup per function: rec = centre, exponents
 // [3], every function's coefficients [3] in the order s; x, y, z; xx, yy, zz,
 // xy, xz, yz.
-template <int TW>
+template <int TW, bool kMoved>
 __device__ __forceinline__ void rows64_shell(const double *rec, int packed, double rx, double ry, double rz, double *chi)
 {
   constexpr int D = rows64_pitch(TW);
   chi += (size_t)(packed & 0xff) * D;
   const int kind = packed >> 16;
   if (kind == kR64Any) {
-    rows64_shell_any<TW>(rec, (packed >> 8) & 0xff, rx, ry, rz, chi);
+    rows64_shell_any<TW, kMoved>(rec, (packed >> 8) & 0xff, rx, ry, rz, chi);
     return;
   }
   Rows64Radial R;
   R.x = rx - rec[0];
   R.y = ry - rec[1];
   R.z = rz - rec[2];
-  const double r2 = R.x * R.x + R.y * R.y + R.z * R.z;
-  const double Lf = 4.0 * kind + 6.0, r2x4 = 4.0 * r2;
+  const double r2 = rows64_r2(R.x, R.y, R.z);
+  const double Lf = 4.0 * kind + 6.0, r2x4 = rows64_r2x4<kMoved>(R.x, R.y, R.z, r2);
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const double a = rec[3 + i];
-    R.e0[i] = exp(-a * r2);
-    R.e1[i] = R.e0[i] * a;
-    R.el[i] = R.e1[i] * fma(r2x4, a, -Lf);
+    R.a[i] = rec[3 + i];
+    R.e[i] = exp(-R.a[i] * r2);
+    R.l[i] = R.a[i] * fma(r2x4, R.a[i], -Lf);
   }
   const double *c = rec + 6;
   if (kind == 0) {

@@ -141,7 +141,9 @@ struct SweepShared {
   static constexpr int kLdB = 8 * kTiles + 4;          // as rows64: 4 mod 8
   static constexpr int kLdR = G + 1;                   // orbitals of a row, zero beyond the spin's
   static constexpr int kSums = 9;
-  static constexpr int kChi = kChunk * kLdA > TW * G * G ? kChunk * kLdA : TW * G * G;
+  // (with room for a shell cut by a chunk's end on either side)
+  static constexpr int kRowsA = (kChunk + (G == 16 ? 2 * kR64Lead : 0)) * kLdA;
+  static constexpr int kChi = ((kRowsA > TW * G * G ? kRowsA : TW * G * G) + 2 * TW - 1) / (2 * TW) * (2 * TW);
   static_assert(kChi % (2 * TW) == 0 && kChi / TW >= G * G, "a walker's inverse in its part of the chunk, 16-byte aligned");
   static constexpr int kC = kChunk * kLdB;
   static constexpr int kPos = kChi + 2 * kC;
@@ -629,11 +631,11 @@ __global__ void __launch_bounds__(TW * G, G == 8 ? 4 : 2)
 #pragma unroll 1
         for (int i = 2 * warp + lane / TW; i < ch.x; i += 2 * kWarps) {
           const double head = rec[i];
-          rows64_shell<TW>(rec + __double2hiint(head), __double2loint(head), rx, ry, rz, chi + lw);
+          rows64_shell<TW, true>(rec + __double2hiint(head), __double2loint(head), rx, ry, rz, chi + lw);
         }
         // padding functions: their coefficients are zero, their values must be finite
         for (int i = (ch.z & 0xffff) * 5 * TW + tid; i < padded * 5 * TW; i += kThreads)
-          chi[i / (5 * TW) * Sh::kLdA + i % (5 * TW)] = 0.0;
+          chi[(T.lead + i / (5 * TW)) * Sh::kLdA + i % (5 * TW)] = 0.0;
       }
       __syncthreads();
       // (a warp's two tiles side by side: their chains overlap)
@@ -641,7 +643,7 @@ __global__ void __launch_bounds__(TW * G, G == 8 ? 4 : 2)
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const int i = warp + j * kWarps;
-        ap[j] = chi + t * Sh::kLdA + 16 * (i % kMT) + g;
+        ap[j] = chi + (T.lead + t) * Sh::kLdA + 16 * (i % kMT) + g;
         bp[j] = Cs + (k & 1) * Sh::kC + t * Sh::kLdB + 8 * (i / kMT) + g;
       }
       for (int kk = 0; kk < padded; kk += 8) {
