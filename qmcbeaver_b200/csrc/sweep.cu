@@ -10,8 +10,8 @@
 //   rows   one walker per half-warp lane: proposals, then the basis shells of
 //          the 16 walkers (a shell per half-warp) and their contraction on the FP64 tensor pipe, as
 //          rows64.cu, the five orbital rows left in shared memory
-//   move   G = 8 or 16 lanes per walker, lane c owning electron c of each
-//          spin and column c of the moved spin's inverse in registers:
+//   move   G = 8 or 16 lanes per walker, lane c owning electrons c and
+//          G + c, and in registers the moved spin's column of one of them:
 //          Jastrow and potential changes, Sherman-Morrison update, ratio
 //          sums, psi quantities, drift, acceptance and reweight, write back
 //
@@ -19,6 +19,16 @@
 // 32 lanes repeat, on warp reductions and on loops over 15 columns or 6 nuclei
 // with idle lanes; with two or four walkers per warp those are shared, and
 // the 3 to 8 sums of a stage go through one transposing reduction.
+//
+// Everything a chain goes on from (rows, inverses, ratio sums, pair sums,
+// drifts) rounds as in k_move: the same operations, and sums over lanes in the
+// order of its 32 lanes, which a lane here takes two (G = 16) or up to four of.
+// A walker next to a node amplifies a rounding by 1e6 and more until the next
+// refresh, so sums in any other order showed as 1e-8 of single local energies.
+// (The laplacian's sum over the columns and the acceptance's exponents, which
+// feed nothing back, add in the lanes' own order, and so does the one sum of
+// the drift limited by a common factor, qf_mod 1.)  150 steps of 16,384 walkers
+// of 30 electrons take 16.7 ms so, 16.0 with sums in the cheapest order.
 //
 // Bound by the latency of a step's chain of phases (30 electrons: 40 k cycles
 // with one CTA per SM -- proposals 1, basis 7.5, products 6, pair terms 3,
@@ -29,7 +39,7 @@
 // registers a thread; with 223 KB of shared memory the L1 is small, so spilled
 // registers cost L2 latencies and the column of the inverse leaves the
 // registers for the ratio sums.  30 electrons, 15,710 walkers: 225 us a step
-// by the move kernel, 84 here; 10 electrons, 100 walkers: 18 and 9.
+// by the move kernel, 90 here; 10 electrons, 100 walkers: 18 and 9.
 #include "rows64_device.cuh"
 #include "sweep.h"
 
@@ -50,26 +60,38 @@ __device__ __forceinline__ double group_sum(double v, unsigned gm)
   return v;
 }
 
-// Sums of eight values over the group at once: lane c returns the total of
-// v[c % 8].  Each of the first three exchanges halves the values a lane keeps.
+// Sums of eight values over the group at once: a lane returns one total
+// (group_total).  The widest exchange first, as group_sum and
+// warp_sum, so that every total has their bits; each of the first three
+// exchanges halves the values a lane keeps.
 template <int G>
 __device__ __forceinline__ double group_sum8(const double v[8], int c, unsigned gm)
 {
   double a[4], b[2];
 #pragma unroll
   for (int k = 0; k < 4; k++) {
-    const double keep = c & 1 ? v[2 * k + 1] : v[2 * k], give = c & 1 ? v[2 * k] : v[2 * k + 1];
-    a[k] = keep + __shfl_xor_sync(gm, give, 1, G);
+    const bool hi = c & (G / 2);
+    const double keep = hi ? v[4 + k] : v[k], give = hi ? v[k] : v[4 + k];
+    a[k] = keep + __shfl_xor_sync(gm, give, G / 2, G);
   }
 #pragma unroll
   for (int k = 0; k < 2; k++) {
-    const double keep = c & 2 ? a[2 * k + 1] : a[2 * k], give = c & 2 ? a[2 * k] : a[2 * k + 1];
-    b[k] = keep + __shfl_xor_sync(gm, give, 2, G);
+    const bool hi = c & (G / 4);
+    const double keep = hi ? a[2 + k] : a[k], give = hi ? a[k] : a[2 + k];
+    b[k] = keep + __shfl_xor_sync(gm, give, G / 4, G);
   }
-  const double keep = c & 4 ? b[1] : b[0], give = c & 4 ? b[0] : b[1];
-  double s = keep + __shfl_xor_sync(gm, give, 4, G);
-  if (G == 16) s += __shfl_xor_sync(gm, s, 8, G);
+  const bool hi = c & (G / 8);
+  const double keep = hi ? b[1] : b[0], give = hi ? b[0] : b[1];
+  double s = keep + __shfl_xor_sync(gm, give, G / 8, G);
+  if (G == 16) s += __shfl_xor_sync(gm, s, 1, G);
   return s;
+}
+// The total of v[k] in every lane: it is with the lanes whose three leading
+// bits are k's.
+template <int G>
+__device__ __forceinline__ double group_total(double sums, int k, unsigned gm)
+{
+  return group_get<G>(sums, k * (G / 8), gm);
 }
 
 // The general correlation functions out of line (the closed form stays inline).
@@ -105,15 +127,14 @@ __device__ __forceinline__ void pair_change(const DevSys &S, int f, double k, bo
                                             const double rn[3], const double P[3], double &dinv, double &dU,
                                             double &dUxx, double v[3])
 {
-  double xo[3], xn[3], r2o = 0.0, r2n = 0.0;
+  double xo[3], xn[3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
     // a lane without a pair computes at distance sqrt(3) and drops the result
     xo[d] = on ? ro[d] - P[d] : 1.0;
     xn[d] = on ? rn[d] - P[d] : 1.0;
-    r2o = fma(xo[d], xo[d], r2o);
-    r2n = fma(xn[d], xn[d], r2n);
   }
+  const double r2o = rows64_r2(xo[0], xo[1], xo[2]), r2n = rows64_r2(xn[0], xn[1], xn[2]);
   const double io = rsqrt(r2o), in_ = rsqrt(r2n);
   dinv = on ? in_ - io : 0.0;
   const bool corr = on && f >= 0;
@@ -122,7 +143,7 @@ __device__ __forceinline__ void pair_change(const DevSys &S, int f, double k, bo
   pair_function(S, f < 0 ? 0 : f, r2n * in_, un, dun, d2un);
   const double sn = corr ? dun * in_ : 0.0, so = corr ? duo * io : 0.0;
   dU += corr ? un - uo : 0.0;
-  dUxx += corr ? k * ((2.0 * sn + d2un) - (2.0 * so + d2uo)) : 0.0;
+  dUxx += corr ? k * ((2.0 * in_ * dun + d2un) - (2.0 * io * duo + d2uo)) : 0.0;
 #pragma unroll
   for (int d = 0; d < 3; d++) v[d] = sn * xn[d] - so * xo[d];
 }
@@ -154,12 +175,24 @@ struct SweepShared {
 // a walker's staged arrays: positions, then gradD .. scalars as in its block
 __host__ __device__ inline int sweep_walker_doubles(const Layout &L) { return L.mv_r + L.mv_tail; }
 
+// The last orbitals of the slices in which the move kernel's 32 lanes share a
+// spin's ratio sums.
+__device__ __forceinline__ unsigned slice_ends_of(int n)
+{
+  unsigned ends = 0;
+  if (n > 0) {
+    const int slices = 32 / n;
+    for (int s = 1; s <= slices; s++) ends |= 1u << n * s / slices >> 1;
+  }
+  return ends;
+}
+
 // One move of the group's walker (list entry wi, tile index gi) from the
 // rows in shared memory; lane c of the group.
 template <bool kMetropolis, int G>
 __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, const RunCfg &cfg, double *blk, int wi,
                                            int gi, int c, unsigned gm, const MoveArgs &mv, const EnergyCtl *ectl,
-                                           double *sm, const EvalOut &out)
+                                           double *sm, unsigned slice_ends, const EvalOut &out)
 {
   using Sh = SweepShared<G>;
   const int N = S.N, e = mv.e, sp = e < S.na ? 0 : 1;
@@ -168,10 +201,11 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   double *sR = sm + Sh::kWalk + (size_t)gi * sweep_walker_doubles(L), *sT = sR + L.mv_r;
   double *sUx = sT + (L.Ux - L.gradD), *smg = sT + (L.mgrad - L.gradD), *sc = sT + (L.sc - L.gradD);
   double *sInv = sm + (size_t)gi * (Sh::kChi / TW);    // the moved spin's inverse, updated in place
-  const int idx[2] = {c, S.na + c};                    // this lane's electrons
-  const bool has[2] = {c < S.na, c < S.nb};
-  const bool mine = c < n;                             // a column of the moved spin
-  const int cc = mine ? c : 0;
+  const int idx[2] = {c, G + c};                       // this lane's electrons
+  const bool has[2] = {idx[0] < N, idx[1] < N};
+  const int col = (c - base) & (G - 1);                // the moved spin's column of one of them,
+  const bool mine = col < n;                           // or none
+  const int cc = mine ? col : 0;
 
   // exponent sum of G(R -> R'): the displacement and, as the reference, the
   // drift of the electrons that stay (QMcBeaver/src/QMCWalker.cpp:383-388)
@@ -197,33 +231,49 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
       ro[d] = sR[3 * e + d];
       rn[d] = sm[Sh::kPos + TW * d + gi];
     }
-    double dU = 0.0, dUxx = 0.0, dVee = 0.0, dVen = 0.0, ge[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int s = 0; s < 2; s++) {
+    // the lanes l = c, G + c (and from 2 G on, for more nuclei than that) of
+    // jastrow_pe_move_warp: electron l, then nuclei l, l + 32, ..
+    double u[7];
+    const auto electron = [&](int s, double w[7]) {
       const double *r = sR + (has[s] ? 3 * idx[s] : 0), P[3] = {r[0], r[1], r[2]};
-      double dinv;
-      pair_change(S, s != sp ? S.ee[0] : s == 0 ? S.ee[1] : S.ee[2], 2.0, has[s] && idx[s] != e, ro, rn, P, dinv, dU,
-                  dUxx, vx[s]);
-      dVee += dinv;
+      w[0] = w[1] = 0.0;
+      pair_change(S, (idx[s] < S.na ? 0 : 1) != sp ? S.ee[0] : sp == 0 ? S.ee[1] : S.ee[2], 2.0,
+                  has[s] && idx[s] != e, ro, rn, P, w[2], w[0], w[1], vx[s]);
+      w[3] = 0.0;
 #pragma unroll
-      for (int d = 0; d < 3; d++) ge[d] += vx[s][d];
+      for (int d = 0; d < 3; d++) w[4 + d] = vx[s][d];
+    };
+    const auto nuclei = [&](int l0, double w[7]) {
+      for (int A0 = l0; A0 < S.M; A0 += 32) {
+        const int A = A0 + c < S.M ? A0 + c : 0;
+        const double4 P = S.nuc[A];
+        const double p[3] = {P.x, P.y, P.z};
+        double v[3], dinv;
+        pair_change(S, S.en[sp][A], 1.0, A0 + c < S.M, ro, rn, p, dinv, w[0], w[1], v);
+        w[3] -= P.w * dinv;
+#pragma unroll
+        for (int d = 0; d < 3; d++) w[4 + d] += v[d];
+      }
+    };
+    electron(0, s8);
+    electron(1, u);
+    nuclei(0, s8);
+    if (S.M > G) nuclei(G, u);
+    if (G == 8 && S.M > 2 * G) {
+      double w[7];
+#pragma unroll
+      for (int k = 0; k < 7; k++) w[k] = 0.0;
+      nuclei(2 * G, w);
+#pragma unroll
+      for (int k = 0; k < 7; k++) s8[k] += w[k];
+#pragma unroll
+      for (int k = 0; k < 7; k++) w[k] = 0.0;
+      nuclei(3 * G, w);
+#pragma unroll
+      for (int k = 0; k < 7; k++) u[k] += w[k];
     }
-    for (int A0 = 0; A0 < S.M; A0 += G) {
-      const int A = A0 + c < S.M ? A0 + c : 0;
-      const double4 P = S.nuc[A];
-      const double p[3] = {P.x, P.y, P.z};
-      double v[3], dinv;
-      pair_change(S, S.en[sp][A], 1.0, A0 + c < S.M, ro, rn, p, dinv, dU, dUxx, v);
-      dVen -= P.w * dinv;
 #pragma unroll
-      for (int d = 0; d < 3; d++) ge[d] += v[d];
-    }
-    s8[0] = dU;
-    s8[1] = dUxx;
-    s8[2] = dVee;
-    s8[3] = dVen;
-#pragma unroll
-    for (int d = 0; d < 3; d++) s8[4 + d] = ge[d];
+    for (int k = 0; k < 7; k++) s8[k] += u[k];
     s8[7] = gf;
   }
   const double sums1 = group_sum8<G>(s8, c, gm);
@@ -235,16 +285,15 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   double inv[G];
 #pragma unroll
   for (int o = 0; o < G; o++) inv[o] = o < n ? sInv[o * n + cc] : 0.0;
-  double dot4[4] = {0.0, 0.0, 0.0, 0.0};
+  const double ratio = group_sum<G>(c < n ? D[c] * sInv[c * n + el] : 0.0, gm);
+  double dot = 0.0;
 #pragma unroll
-  for (int o = 0; o < G; o++) dot4[o & 3] = fma(D[o], inv[o], dot4[o & 3]);
-  const double dot = (dot4[0] + dot4[1]) + (dot4[2] + dot4[3]);
-  const double ratio = group_get<G>(dot, el, gm);
+  for (int o = 0; o < G; o++) dot = fma(D[o], inv[o], dot);
   bool bad = !(ratio != 0.0) || !isfinite(ratio);
   const double q = 1.0 / ratio;
   {
     // inv - vc * (old column of the moved electron), its own column inv * q
-    const double vc = c == el ? 0.0 : dot * q, f = c == el ? q : 1.0;
+    const double vc = col == el ? 0.0 : dot * q, f = col == el ? q : 1.0;
 #pragma unroll
     for (int o = 0; o < G; o++) inv[o] = fma(-vc, o < n ? sInv[o * n + el] : 0.0, f * inv[o]);
   }
@@ -253,51 +302,64 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   if (mine) {
 #pragma unroll
     for (int o = 0; o < G; o++)
-      if (o < n) sInv[o * n + c] = inv[o];
+      if (o < n) sInv[o * n + col] = inv[o];
   }
 
   // ---- ratio sums of the moved spin (QMcBeaver/src/QMCSlater.cpp:741-762):
   //      this lane's column of the inverse with its derivative columns (the
-  //      moved electron's from the new rows).  The rows are read once per move
+  //      moved electron's from the new rows), added up slice by slice as the
+  //      move kernel's lanes do.  The rows are read once per move
   //      (from L2), eight orbitals' loads in flight; addresses past the
   //      spin's orbitals are clamped and their terms dropped.
   double lp = 0.0, gn[3] = {0.0, 0.0, 0.0};
   {
     const Deriv4<double> *D4 = (const Deriv4<double> *)(blk + L.D4[sp]) + cc;
-    const bool own = c == el;
+    const bool own = col == el;
     constexpr int kB = 8;
+    // slice by slice for the larger spins (2 or 3 of up to 8 orbitals), the
+    // whole column in one batch for the smaller (4 or more of up to 2)
+    const int slices = G == 16 ? 32 / n : 1;
 #pragma unroll 1
-    for (int o0 = 0; o0 < n; o0 += kB) {
-      Deriv4<double> g[kB];
+    for (int s = 0; s < slices; s++) {
+      const int oa = G == 16 ? n * s / slices : 0, ob = G == 16 ? n * (s + 1) / slices : n;
+      if (oa == ob) continue;
+      Deriv4<double> g[kB], part = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-      for (int u = 0; u < kB; u++) g[u] = ld_deriv<false>(D4 + min(o0 + u, n - 1) * n);
+      for (int u = 0; u < kB; u++) g[u] = ld_deriv<false>(D4 + min(oa + u, ob - 1) * n);
 #pragma unroll
       for (int u = 0; u < kB; u++) {
-        const int o = min(o0 + u, n - 1);
-        const double iv = o0 + u < n ? sInv[o * n + cc] : 0.0;
+        const int o = min(oa + u, ob - 1);
+        const double iv = oa + u < ob ? sInv[o * n + cc] : 0.0;
         const double *Do = D + o;
-        gn[0] = fma(own ? Do[Sh::kLdR] : g[u].x, iv, gn[0]);
-        gn[1] = fma(own ? Do[2 * Sh::kLdR] : g[u].y, iv, gn[1]);
-        gn[2] = fma(own ? Do[3 * Sh::kLdR] : g[u].z, iv, gn[2]);
-        lp = fma(own ? Do[4 * Sh::kLdR] : g[u].l, iv, lp);
+        part.x = fma(own ? Do[Sh::kLdR] : g[u].x, iv, part.x);
+        part.y = fma(own ? Do[2 * Sh::kLdR] : g[u].y, iv, part.y);
+        part.z = fma(own ? Do[3 * Sh::kLdR] : g[u].z, iv, part.z);
+        part.l = fma(own ? Do[4 * Sh::kLdR] : g[u].l, iv, part.l);
+        if (G == 8 ? slice_ends >> u & 1 : u == kB - 1) {  // the same in the whole block
+          gn[0] += part.x;
+          gn[1] += part.y;
+          gn[2] += part.z;
+          lp += part.l;
+          part = {0.0, 0.0, 0.0, 0.0};
+        }
       }
     }
     lp = mine ? lp : 0.0;
   }
 
   // ---- psi quantities (psi_lap_warp) and the modified drift (qf_modify_warp)
-  double gr[2][3], mg[2][3], part = 0.0, pu = 0.0, pm = 0.0, pr = 0.0;
+  double gr[2][3], mg[2][3], part[2] = {0.0, 0.0}, pu = 0.0, pm = 0.0, pr = 0.0;
   double R[2][3], Ux[2][3], gD[2][3];
 #pragma unroll
   for (int d = 0; d < 3; d++) {
-    const double ge = group_get<G>(sums1, 4 + d, gm);
+    const double ge = group_total<G>(sums1, 4 + d, gm);
 #pragma unroll
     for (int s = 0; s < 2; s++) {
       const int i = has[s] ? 3 * idx[s] + d : d;
-      const bool me = s == sp && c == el;
-      const double u = sUx[i] + (me ? ge : -vx[s][d]), g = s == sp ? gn[d] : sT[i];
+      const bool me = idx[s] == e;
+      const double u = sUx[i] + (me ? ge : -vx[s][d]);
       Ux[s][d] = has[s] ? u : 0.0;
-      gD[s][d] = has[s] ? g : 0.0;
+      gD[s][d] = has[s] ? (idx[s] == base + col && mine ? gn[d] : sT[i]) : 0.0;
       R[s][d] = me ? sm[Sh::kPos + TW * d + gi] : sR[i];
     }
   }
@@ -307,8 +369,8 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
     for (int d = 0; d < 3; d++) {
       const double x = gD[s][d], u = Ux[s][d];
       gr[s][d] = x + u;
-      part += u * x * 2.0;
-      part += u * u;
+      part[s] += u * x * 2.0;
+      part[s] += u * u;
       pu += gr[s][d] * gr[s][d];
     }
   double factor[2] = {1.0, 1.0};
@@ -365,19 +427,19 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
           pr += tt * tt;
         }
   }
-  const double t8[8] = {lp, part, pm, pu, pr, 0.0, 0.0, 0.0};
+  const double t8[8] = {lp, part[0] + part[1], pm, pu, pr, 0.0, 0.0, 0.0};
   const double sums2 = group_sum8<G>(t8, c, gm);
-  const double lapR = group_get<G>(sums2, 0, gm);
+  const double lapR = group_total<G>(sums2, 0, gm);
   double Dxx = 0.0;
   if (S.na > 0) Dxx += sp == 0 ? lapR : sc[SC_LAPR_A];
   if (S.nb > 0) Dxx += sp == 1 ? lapR : sc[SC_LAPR_B];
-  const double dU = group_get<G>(sums1, 0, gm);
-  const double U_new = sc[SC_U] + dU, Uxx_new = sc[SC_UXX] + group_get<G>(sums1, 1, gm);
-  const double lap = Dxx + Uxx_new + group_get<G>(sums2, 1, gm);
-  const double lm = sqrt(group_get<G>(sums2, 2, gm)), lu = sqrt(group_get<G>(sums2, 3, gm));
+  const double dU = group_total<G>(sums1, 0, gm);
+  const double U_new = sc[SC_U] + dU, Uxx_new = sc[SC_UXX] + group_total<G>(sums1, 1, gm);
+  const double lap = Dxx + Uxx_new + group_total<G>(sums2, 1, gm);
+  const double lm = sqrt(group_total<G>(sums2, 2, gm)), lu = sqrt(group_total<G>(sums2, 3, gm));
   const double modratio = lm / lu;
   if (isnan(lm) || isnan(lu) || isnan(modratio) || lu == 0.0) bad = true;
-  const double Vee = sc[SC_VEE] + group_get<G>(sums1, 2, gm), Ven = sc[SC_VEN] + group_get<G>(sums1, 3, gm);
+  const double Vee = sc[SC_VEE] + group_total<G>(sums1, 2, gm), Ven = sc[SC_VEN] + group_total<G>(sums1, 3, gm);
   const double PE = S.Pnn + Vee + Ven;
   const double EL = -0.5 * lap + PE;
   if (isnan(EL)) bad = true;
@@ -390,13 +452,13 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   if (kMetropolis) {
     double log_g = 0.0;
     if (cfg.sampling == 1) {
-      double g_fwd = group_get<G>(sums1, 7, gm);
+      double g_fwd = group_total<G>(sums1, 7, gm);
 #pragma unroll
       for (int d = 0; d < 3; d++) {
         const double x = sm[Sh::kPos + (3 + d) * TW + gi];
         g_fwd += x * x;
       }
-      log_g = -(group_get<G>(sums2, 4, gm) - g_fwd) / (2.0 * cfg.dt);
+      log_g = -(group_total<G>(sums2, 4, gm) - g_fwd) / (2.0 * cfg.dt);
     }
     MoveTally ty;
     double ro[3], rn[3];
@@ -455,7 +517,7 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
   if (accept) {
     double *Inv = blk + L.Inv[sp];
     for (int i = c; i < n * n; i += G) Inv[i] = sInv[i];
-    if (mine) {
+    if (c < n) {
       // lane c writes orbital c of the moved electron's new rows
       blk[L.Dv[sp] + el * n + c] = D[c];
       ((Deriv4<double> *)(blk + L.D4[sp]))[c * n + el] = {D[Sh::kLdR + c], D[2 * Sh::kLdR + c], D[3 * Sh::kLdR + c],
@@ -467,10 +529,8 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
 #pragma unroll
         for (int d = 0; d < 3; d++) {
           const int t = 3 * idx[s] + d;
-          if (s == sp) {
-            sT[t] = gD[s][d];
-            if (c == el) sR[t] = R[s][d];
-          }
+          sT[t] = gD[s][d];  // (the other spin's as they were)
+          if (idx[s] == e) sR[t] = R[s][d];
           sUx[t] = Ux[s][d];
           smg[t] = mg[s][d];
         }
@@ -571,6 +631,7 @@ __global__ void __launch_bounds__(TW * G, G == 8 ? 4 : 2)
   cp_async_commit();
   __syncthreads();
   const int nsteps = kMetropolis ? a.nsteps : 1;
+  const unsigned ends[2] = {slice_ends_of(S.na), slice_ends_of(S.nb)};
   MoveArgs mv{};
   {
     const int e0 = kMetropolis ? a.step0 % S.N : a.e;
@@ -686,7 +747,7 @@ __global__ void __launch_bounds__(TW * G, G == 8 ? 4 : 2)
     __syncthreads();
 
     // ---- moves
-    if (active) sweep_move<kMetropolis, G>(S, L, cfg, blk, wi, gi, c, gm, mv, ectl, sm, out);
+    if (active) sweep_move<kMetropolis, G>(S, L, cfg, blk, wi, gi, c, gm, mv, ectl, sm, ends[sp], out);
     // the walkers' new state is read by other lanes of this CTA next step
     __syncthreads();
   }
