@@ -474,10 +474,15 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
     // the functions of a complete shell in the order of its kind
     const int order[3][6] = {{0}, {1, 1 << 8, 1 << 16}, {2, 2 << 8, 2 << 16, 1 | 1 << 8, 1 | 1 << 16, 1 << 8 | 1 << 16}};
     if (L <= 2 && np <= 3 && nmem == (L + 1) * (L + 2) / 2) {
-      for (int m = 0; m < nmem; m++)
+      // (every component once: a run of px, px, py of two contractions over the
+      // same exponents is none)
+      bool complete = true;
+      for (int m = 0; m < nmem && complete; m++) {
         for (int k = sh.y; k < sh.y + nmem; k++)
           if (fn[k].x == order[L][m]) it.members.push_back(k);
-      if ((int)it.members.size() == nmem) {
+        complete = (int)it.members.size() == m + 1;
+      }
+      if (complete) {
         it.kind = L;
         items.push_back(it);
         continue;
