@@ -200,11 +200,15 @@ static int fail(qmcb_handle *h, int code, const std::string &msg)
   return code;
 }
 
+// (a failed launch's error is also the thread's last one: taken back, so that
+// the next call does not report it again)
 #define CK(call)                                                                       \
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
-    if (e_ != cudaSuccess)                                                             \
+    if (e_ != cudaSuccess) {                                                           \
+      cudaGetLastError();                                                              \
       return fail(h, QMCB_E_CUDA, std::string(#call ": ") + cudaGetErrorString(e_));   \
+    }                                                                                  \
   } while (0)
 
 static RunCfg make_cfg(const qmcb_run_params &p)
@@ -428,16 +432,16 @@ static bool move_dense_wins(const qmcb_handle *h, bool rows, int n)
 
 // One launch of the single-determinant move kernel in the walker state's
 // precision, with the cusp / three-body code only when the system has them.
-static void launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extras, const dim3 &g, const dim3 &b,
-                          size_t sm, cudaStream_t st, const RunCfg &cfg, const int *slots, int num, const int *d_num,
-                          const double *R_in, const MoveArgs &mv, const EvalOut &o)
+static cudaError_t launch_move_g(qmcb_handle *h, bool metropolis, bool mixed, bool extras, const dim3 &g, const dim3 &b,
+                                 size_t sm, cudaStream_t st, const RunCfg &cfg, const int *slots, int num, const int *d_num,
+                                 const double *R_in, const MoveArgs &mv, const EvalOut &o)
 {
   // with rows from a batched kernel the scratch has no basis rows
   const Layout &L = mv.rows ? h->lay_rows : h->lay;
   // (the walkers of a run change with branching; their first number decides)
   const bool dense = extras && !mixed && move_dense_wins(h, mv.rows != nullptr, d_num ? h->n_start : num);
-  launch_kernel(dense ? move_dense_fn(metropolis) : move_fn(metropolis, mixed, extras, h->ginv), g, b, sm, st, h->sys, L,
-                cfg, h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
+  return launch_kernel(dense ? move_dense_fn(metropolis) : move_fn(metropolis, mixed, extras, h->ginv), g, b, sm, st,
+                       h->sys, L, cfg, h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
 }
 
 // The chunks of k_rows64 (struct Rows64), filled in the order of the basis
@@ -641,8 +645,8 @@ static bool batched_rows(const qmcb_handle *h)
 // rows modes) into h->d_rows_out: proposal + basis operand planes, then the
 // contraction; prof: record the two kernels' times (not under stream capture).
 template <bool kMetropolis>
-static void launch_rows(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
-                        const int *d_num, const double *R_in, const MoveArgs &mv, bool extras, bool prof)
+static cudaError_t launch_rows(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
+                               const int *d_num, const double *R_in, const MoveArgs &mv, bool extras, bool prof)
 {
   const int prec = h->params.precision;
   const int sp = mv.e < h->sys.na ? 0 : 1, n = sp ? h->sys.nb : h->sys.na;
@@ -695,6 +699,7 @@ static void launch_rows(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
   }
   h->rows_n = n;
   h->rows_num = cap;
+  return cudaGetLastError();
 }
 
 // One single-electron move of list entries [0, num) (d_num: device count,
@@ -702,52 +707,56 @@ static void launch_rows(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
 // launches: proposal + basis digits, the tensor-core contraction, the move
 // kernel on the rows; else the move kernel alone.
 template <bool kMetropolis>
-static void launch_move(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
-                        const int *d_num, const double *R_in, MoveArgs mv, EvalOut o)
+static cudaError_t launch_move(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
+                               const int *d_num, const double *R_in, MoveArgs mv, EvalOut o)
 {
   if (!kMetropolis && sweep_moves(h)) {
     SweepArgs a{};
     a.e = mv.e;
     a.rin_moved = mv.rin_moved;
     ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-    sweep_launch(false, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num, R_in, a, h->d_ectl,
-                 h->d_stats, o);
+    const cudaError_t err = sweep_launch(false, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num,
+                                         R_in, a, h->d_ectl, h->d_stats, o);
     ps.end(st);
-    return;
+    return err;
   }
   // the Umrigar93 move is compiled only into the extras instantiation
   const bool extras = h->extras || (kMetropolis && cfg.sampling == QMCB_UMRIGAR93_IMPORTANCE_SAMPLING);
   if (rows_mode(h->params.precision)) {
-    launch_rows<kMetropolis>(h, cap, st, cfg, slots, num, d_num, R_in, mv, extras, true);
+    cudaError_t err = launch_rows<kMetropolis>(h, cap, st, cfg, slots, num, d_num, R_in, mv, extras, true);
+    if (err != cudaSuccess) return err;
     mv.rows = h->d_rows_out;
     const dim3 g((cap + h->wpb_rows - 1) / h->wpb_rows), b(32 * h->wpb_rows);
     ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-    launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
+    err = launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
     ps.end(st);
-    return;
+    return err;
   }
   // (the rows buffer is the handle's: calls for disjoint walkers on callers'
   // streams may overlap, and evaluate their rows in the move kernel)
   if (rows64_moves(h, cap) && st == h->stream) {
+    cudaError_t err;
     {
       ProfScope ps(h, QMCB_KERNEL_ROWS_PREP, st);
-      rows64_launch(kMetropolis ? R64_PROPOSE : R64_GIVEN, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num,
-                    d_num, R_in, mv, mv.e < h->sys.na ? 0 : 1, h->d_rows64);
+      err = rows64_launch(kMetropolis ? R64_PROPOSE : R64_GIVEN, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st,
+                          slots, num, d_num, R_in, mv, mv.e < h->sys.na ? 0 : 1, h->d_rows64);
       ps.end(st);
     }
+    if (err != cudaSuccess) return err;
     mv.rows = h->d_rows64;
     const dim3 g((cap + h->wpb_rows - 1) / h->wpb_rows), b(32 * h->wpb_rows);
     ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-    launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
+    err = launch_move_g(h, kMetropolis, false, extras, g, b, h->smem_rows, st, cfg, slots, num, d_num, R_in, mv, o);
     ps.end(st);
-    return;
+    return err;
   }
   const dim3 g((cap + h->wpb_move - 1) / h->wpb_move), b(32 * h->wpb_move);
   const size_t sm = h->smem_move;
   ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-  launch_move_g(h, kMetropolis, h->params.precision == QMCB_PREC_MIXED, extras, g, b, sm, st, cfg, slots, num, d_num,
-                R_in, mv, o);
+  const cudaError_t err = launch_move_g(h, kMetropolis, h->params.precision == QMCB_PREC_MIXED, extras, g, b, sm, st, cfg,
+                                        slots, num, d_num, R_in, mv, o);
   ps.end(st);
+  return err;
 }
 
 // ---------------------------------------------------------------------------
@@ -1626,8 +1635,8 @@ int qmcb_synchronize(qmcb_handle *h)
 }
 
 // One launch of the single-determinant full-evaluation / refresh kernel.
-static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
-                        const int *d_num, const double *R_in, int do_basis, EvalOut o)
+static cudaError_t launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
+                               const int *d_num, const double *R_in, int do_basis, EvalOut o)
 {
   // list entries [0, num) (d_num: device count), grid sized for `cap`;
   // the refresh (do_basis = 0, 2) runs with its smaller per-warp scratch
@@ -1638,14 +1647,18 @@ static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
     // one warp a walker and this way: 3 electrons 24, 71 and 25, 41; 10: 79,
     // 254 and 37, 84; 30: 301, 1,262 and 66, 331; 100: 5,083, 38,592 and 357,
     // 6,673.  (The cusp replacement works on rows before they are stored.)
-    for (int sp = 0; sp < 2; sp++)
-      rows64_launch(R64_ALL, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num, d_num, R_in, MoveArgs{}, sp,
-                    nullptr);
+    for (int sp = 0; sp < 2; sp++) {
+      const cudaError_t err = rows64_launch(R64_ALL, h->sys, h->lay, cfg, h->r64, h->d_state, cap, st, slots, num,
+                                            d_num, R_in, MoveArgs{}, sp, nullptr);
+      if (err != cudaSuccess) return err;
+    }
     do_basis = 0;
   }
   if (!do_basis && h->nmax <= kInvertMax) {
     // the inverses in a kernel of their own (invert.cu), then the rest
-    invert_launch(h->params.precision == QMCB_PREC_MIXED, h->sys, h->lay, h->d_state, cap, st, slots, num, d_num);
+    const cudaError_t err =
+        invert_launch(h->params.precision == QMCB_PREC_MIXED, h->sys, h->lay, h->d_state, cap, st, slots, num, d_num);
+    if (err != cudaSuccess) return err;
     do_basis = 2;
   }
   const int wpb = do_basis == 2 ? kMaxWarpsPerBlock : do_basis ? h->wpb_full : h->wpb_refresh;
@@ -1655,24 +1668,24 @@ static void launch_full(qmcb_handle *h, int cap, cudaStream_t st, const RunCfg &
                                   : h->smem_refresh;
   const bool mixed = h->params.precision == QMCB_PREC_MIXED;
   const bool dense = do_basis == 2 && h->extras && (d_num ? h->n_start : num) > h->rest_wave;
-  launch_kernel(dense ? rest_dense_fn(mixed) : full_fn(mixed, h->extras, do_basis == 2), g, b, sm, st, h->sys, h->lay, cfg,
-                h->d_state, slots, num, d_num, R_in, do_basis, o);
+  return launch_kernel(dense ? rest_dense_fn(mixed) : full_fn(mixed, h->extras, do_basis == 2), g, b, sm, st, h->sys,
+                       h->lay, cfg, h->d_state, slots, num, d_num, R_in, do_basis, o);
 }
 
 // The several-determinant kernels.
-static void launch_full_md(qmcb_handle *h, int blocks, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
-                           const int *d_num, const double *R_in, int do_basis, const EvalOut &o)
+static cudaError_t launch_full_md(qmcb_handle *h, int blocks, cudaStream_t st, const RunCfg &cfg, const int *slots, int num,
+                                  const int *d_num, const double *R_in, int do_basis, const EvalOut &o)
 {
-  launch_kernel(full_md_fn(), dim3(blocks), dim3(32 * h->wpb_full), h->smem_full, st, h->sys, h->lay, cfg, h->d_state,
-                slots, num, d_num, R_in, do_basis, o);
+  return launch_kernel(full_md_fn(), dim3(blocks), dim3(32 * h->wpb_full), h->smem_full, st, h->sys, h->lay, cfg,
+                       h->d_state, slots, num, d_num, R_in, do_basis, o);
 }
 
-static void launch_move_md(qmcb_handle *h, bool metropolis, int blocks, cudaStream_t st, const RunCfg &cfg,
-                           const int *slots, int num, const int *d_num, const double *R_in, const MoveArgs &mv,
-                           const EvalOut &o)
+static cudaError_t launch_move_md(qmcb_handle *h, bool metropolis, int blocks, cudaStream_t st, const RunCfg &cfg,
+                                  const int *slots, int num, const int *d_num, const double *R_in, const MoveArgs &mv,
+                                  const EvalOut &o)
 {
-  launch_kernel(move_md_fn(metropolis), dim3(blocks), dim3(32 * h->wpb_move), h->smem_move, st, h->sys, h->lay, cfg,
-                h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
+  return launch_kernel(move_md_fn(metropolis), dim3(blocks), dim3(32 * h->wpb_move), h->smem_move, st, h->sys, h->lay,
+                       cfg, h->d_state, slots, num, d_num, R_in, mv, h->d_ectl, h->d_stats, o);
 }
 
 // Device address of a host array that kernels can store into directly:
@@ -1807,27 +1820,25 @@ static int launch_eval(qmcb_handle *h, int which_e, const int *d_slots, int num,
     if (mixed) return fail(h, QMCB_E_ARG, "evaluate: several determinants run in FP64 (precision QMCB_PREC_FP64)");
     if (which_e < 0) {
       int blocks = (num + h->wpb_full - 1) / h->wpb_full;
-      launch_full_md(h, blocks, st, cfg, d_slots, num, nullptr, d_R, 1, o);
+      CK(launch_full_md(h, blocks, st, cfg, d_slots, num, nullptr, d_R, 1, o));
     } else {
       MoveArgs mv{which_e, 0, 0, 0};
       mv.rin_moved = rin_moved;
       int blocks = (num + h->wpb_move - 1) / h->wpb_move;
-      launch_move_md(h, false, blocks, st, cfg, d_slots, num, nullptr, d_R, mv, o);
+      CK(launch_move_md(h, false, blocks, st, cfg, d_slots, num, nullptr, d_R, mv, o));
     }
-    CK(cudaGetLastError());
     if (which_e < 0) h->state_prec = h->params.precision;
     return QMCB_OK;
   }
   if (which_e < 0) {
-    launch_full(h, num, st, cfg, d_slots, num, nullptr, d_R, 1, o);
+    CK(launch_full(h, num, st, cfg, d_slots, num, nullptr, d_R, 1, o));
   } else {
     if (h->state_prec != state_kind(h->params.precision))
       return fail(h, QMCB_E_STATE, "evaluate: walker state was written in another precision; evaluate all electrons first");
     MoveArgs mv{which_e, 0, 0, 0};
     mv.rin_moved = rin_moved;
-    launch_move<false>(h, num, st, cfg, d_slots, num, nullptr, d_R, mv, o);
+    CK(launch_move<false>(h, num, st, cfg, d_slots, num, nullptr, d_R, mv, o));
   }
-  CK(cudaGetLastError());
   if (which_e < 0) h->state_prec = state_kind(h->params.precision);
   return QMCB_OK;
 }
@@ -2007,10 +2018,10 @@ static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int 
       ps.end(st);
     } else if (h->md) {
       ProfScope ps(h, QMCB_KERNEL_MOVE, st);
-      launch_move_md(h, true, blocks, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o);
+      CK(launch_move_md(h, true, blocks, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o));
       ps.end(st);
     } else {
-      launch_move<true>(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o);
+      CK(launch_move<true>(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o));
     }
     if (dmc && mv.e == 0) {
       {
@@ -2035,9 +2046,9 @@ static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int 
       EvalOut o2{};
       ProfScope ps(h, QMCB_KERNEL_REFRESH, st);
       if (h->md)
-        launch_full_md(h, blocks_full, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2);
+        CK(launch_full_md(h, blocks_full, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2));
       else
-        launch_full(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2);
+        CK(launch_full(h, h->max_walkers, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2));
       ps.end(st);
     }
   }
@@ -2362,8 +2373,10 @@ static int gfail(qmcb_group *g, int code, const std::string &msg)
 #define GK(call)                                                                       \
   do {                                                                                 \
     cudaError_t e_ = (call);                                                           \
-    if (e_ != cudaSuccess)                                                             \
+    if (e_ != cudaSuccess) {                                                           \
+      cudaGetLastError();                                                              \
       return gfail(g, QMCB_E_CUDA, std::string(#call ": ") + cudaGetErrorString(e_));  \
+    }                                                                                  \
   } while (0)
 
 static bool member_extras(const qmcb_handle *h)
@@ -2533,8 +2546,8 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
         mv.reweight_on = mv.step >= h->params.reweight_start_step;
         mv.dump = nullptr;
         if (rows_mode(h->params.precision))
-          launch_rows<true>(h, h->max_walkers, h->stream, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, mv,
-                            member_extras(h), false);
+          GK(launch_rows<true>(h, h->max_walkers, h->stream, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, mv,
+                               member_extras(h), false));
         else
           GK(rows64_launch(R64_PROPOSE, h->sys, h->lay, make_cfg(h->params), h->r64, h->d_state, h->max_walkers,
                            h->stream, h->d_live, 0, h->d_ctl, nullptr, mv, mv.e < h->sys.na ? 0 : 1, h->d_rows64));
@@ -2553,9 +2566,9 @@ static int group_enqueue(qmcb_group *g, int c, int n_steps, const int *first_ste
             EvalOut o2{};
             const int blocks_full = (h->max_walkers + h->wpb_full - 1) / h->wpb_full;
             if (h->md)
-              launch_full_md(h, blocks_full, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2);
+              GK(launch_full_md(h, blocks_full, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2));
             else
-              launch_full(h, h->max_walkers, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2);
+              GK(launch_full(h, h->max_walkers, sb, make_cfg(h->params), h->d_live, 0, h->d_ctl, nullptr, 0, o2));
           }
         }
       }

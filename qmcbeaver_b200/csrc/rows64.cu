@@ -39,10 +39,10 @@ static __device__ __noinline__ void rows64_umrigar(const DevSys &S, const RunCfg
 }
 
 // rows[list index][5][n] (R64_PROPOSE, R64_GIVEN), or the walkers' stored
-// Slater values and derivative rows (R64_ALL).  Grid: R64_ALL: x = electrons
-// of the spin x orbital splits (a tile's electrons adjacent, so that their
-// interleaved derivative columns meet in L2), y = tiles of 32 list entries;
-// else x = tiles, y = splits.
+// Slater values and derivative rows (R64_ALL).  Grid: R64_ALL: x = tiles of 32
+// list entries x electrons of the spin x orbital splits (a tile's electrons
+// adjacent, so that their interleaved derivative columns meet in L2; one
+// dimension, since the others end at 65,535 tiles); else x = tiles, y = splits.
 //
 // Per chunk the warps evaluate its shells, meet, multiply, and meet again; the
 // next chunk's coefficients and records land meanwhile.  The two
@@ -64,13 +64,13 @@ __global__ void __launch_bounds__(32 * kR64MTiles *NH, NH == 2 ? 1 : 2)
   constexpr int kWarps = kR64MTiles * NH, kThreads = 32 * kWarps;
   constexpr int kLdB = 8 * NT * NH + 4;
   const int nw = d_num ? *d_num : num;
-  const int w0 = (kMode == R64_ALL ? blockIdx.y : blockIdx.x) * kR64Walkers;
+  const int n = sp ? S.nb : S.na, base = sp ? S.na : 0;
+  const int splits = rows64_splits(n), per_tile = kMode == R64_ALL ? n * splits : 1;
+  const int w0 = blockIdx.x / per_tile * kR64Walkers;
   if (w0 >= nw) return;
   const int lane = lane_id(), warp = threadIdx.x >> 5, tid = threadIdx.x;
-  const int n = sp ? S.nb : S.na, base = sp ? S.na : 0;
-  const int splits = kMode == R64_ALL ? gridDim.x / n : gridDim.y;
   const int split = kMode == R64_ALL ? blockIdx.x % splits : blockIdx.y;
-  const int e = kMode == R64_ALL ? base + blockIdx.x / splits : mv.e;
+  const int e = kMode == R64_ALL ? base + blockIdx.x % per_tile / splits : mv.e;
   double *chi = sm64;                           // [kR64Lead + kR64Chunk][kR64LdA], the chunk from row T.lead
   double *Cs = chi + (kR64Lead + kR64Chunk) * kR64LdA;  // two buffers [kR64Chunk][kLdB]
   double *pos = Cs + 2 * kR64Chunk * kLdB;      // [3][32]
@@ -224,7 +224,7 @@ cudaError_t rows64_launch(Rows64Mode mode, const DevSys &S, const Layout &L, con
   if (n == 0) return cudaSuccess;
   const int nt = rows64_tiles(n), nh = rows64_halves(n), splits = rows64_splits(n);
   const int tiles = (cap + kR64Walkers - 1) / kR64Walkers;
-  const dim3 g = mode == R64_ALL ? dim3(n * splits, tiles) : dim3(tiles, splits);
+  const dim3 g = mode == R64_ALL ? dim3((unsigned)tiles * n * splits) : dim3(tiles, splits);
   const void *fn = mode == R64_ALL       ? rows64_fn<R64_ALL>(nt, nh)
                    : mode == R64_PROPOSE ? rows64_fn<R64_PROPOSE>(nt, nh)
                                          : rows64_fn<R64_GIVEN>(nt, nh);
