@@ -2356,8 +2356,10 @@ struct qmcb_group {
   std::vector<cudaEvent_t> sweep_ev;
   int *d_no_walkers = nullptr;  // control words of an empty walker list
   cudaGraphExec_t gexec = nullptr;  // the last batch's launch sequence
+  // what it was captured for: steps, configuration and, per member, whether it
+  // sweeps (0), moves in its bucket (1) or also branches there (2)
   int g_steps = -1, g_config = -1;
-  std::vector<char> g_sweeps;
+  std::vector<char> g_kinds;
   std::string err;
 };
 
@@ -2766,7 +2768,10 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
   if (!others) {
     // every member runs on its own stream
   } else if (!refresh && !rows_members && n_steps > 0) {
-    if (!(g->gexec && g->g_steps == n_steps && g->g_config == c && g->g_sweeps == g->sweeps)) {
+    std::vector<char> kinds(nm, 0);
+    for (int i = 0; i < nm; i++)
+      if (!g->sweeps[i]) kinds[i] = g->h_gm[i].dmc ? 2 : 1;
+    if (!(g->gexec && g->g_steps == n_steps && g->g_config == c && g->g_kinds == kinds)) {
       if (g->gexec) {
         cudaGraphExecDestroy(g->gexec);
         g->gexec = nullptr;
@@ -2788,7 +2793,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
       }
       g->g_steps = n_steps;
       g->g_config = c;
-      g->g_sweeps = g->sweeps;
+      g->g_kinds = kinds;
     }
     GK(cudaGraphLaunch(g->gexec, st));
   } else {

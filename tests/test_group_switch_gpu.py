@@ -1,0 +1,47 @@
+"""A group whose members' run parameters change between batches of the same
+number of steps: every member follows the chain it follows alone."""
+import numpy as np
+import pytest
+
+from qmcbeaver_b200.api import QMCB200Group
+from qmcbeaver_b200.desc import QMCB_DMC, run_params
+from qmcbeaver_b200.system import make_random_molecule, with_three_body
+from test_group_gpu import _dmc_params, _handles, _params
+
+pytestmark = pytest.mark.gpu
+
+
+def _systems():
+    sizes = [(6, 1, 24, 200), (10, 2, 40, 150), (36, 7, 144, 120)]
+    out = [(make_random_molecule(ne, nn, nb, 5.0 + ne / 10, (1, 6, 7, 8), seed=30 + k), w)
+           for k, (ne, nn, nb, w) in enumerate(sizes)]
+    out[1] = (with_three_body(out[1][0], seed=3), out[1][1])
+    return out
+
+
+def test_vmc_then_dmc_without_refreshes():
+    systems = _systems()
+    solo, grouped = _handles(systems, _params), _handles(systems, _params)
+    g = QMCB200Group(grouped)
+    g.set_config(0)
+    n = 36
+    g.run_steps(0, n)
+    for f in solo:
+        f.run_steps(0, n)
+    for f, h in zip(solo, grouped):
+        e0 = float(np.median(f.get_walkers()["e_local"]))
+        p = _dmc_params(0, e0)
+        p.refresh_interval = 0
+        assert p.run_type == QMCB_DMC
+        f.set_params(p)
+        h.set_params(p)
+    got = g.run_steps(n, n)
+    for f, h, st_g in zip(solo, grouped, got):
+        st = f.run_steps(n, n)
+        assert st_g.n_walkers == st.n_walkers
+        assert st.final_weight > 0  # the last branching pass's sum
+        assert st_g.final_weight == pytest.approx(st.final_weight, rel=1e-9)
+        a, b = f.get_walkers(), h.get_walkers()
+        assert np.array_equal(a["R"], b["R"])
+        assert np.allclose(a["weight"], b["weight"], rtol=1e-9)
+    g.close()
