@@ -1986,7 +1986,9 @@ int qmcb_init_walkers(qmcb_handle *h, int n, const double *R)
 }
 
 // The launches of n_steps Monte Carlo steps on st (dump: see enqueue_steps).
-static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int first_step, int n_steps, double *dump)
+// prof: into the handle's kernel statistics (whoever passes it collects them).
+static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int first_step, int n_steps, double *dump,
+                        bool prof)
 {
   const int blocks = (h->max_walkers + h->wpb_move - 1) / h->wpb_move;
   const int blocks_full = (h->max_walkers + h->wpb_full - 1) / h->wpb_full;
@@ -2012,12 +2014,12 @@ static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int 
            a.nsteps++, s++)
         step++;
       mv.e = step % h->N;
-      ProfScope ps(h, QMCB_KERNEL_MOVE, st);
+      ProfScope ps(h, QMCB_KERNEL_MOVE, st, prof);
       CK(sweep_launch(true, h->sys, h->lay, cfg, h->r64, h->d_state, h->max_walkers, st, h->d_live, 0, h->d_ctl,
                       nullptr, a, h->d_ectl, h->d_stats, o));
       ps.end(st);
     } else if (h->md) {
-      ProfScope ps(h, QMCB_KERNEL_MOVE, st);
+      ProfScope ps(h, QMCB_KERNEL_MOVE, st, prof);
       CK(launch_move_md(h, true, blocks, st, cfg, h->d_live, 0, h->d_ctl, nullptr, mv, o));
       ps.end(st);
     } else {
@@ -2025,26 +2027,26 @@ static int launch_steps(qmcb_handle *h, cudaStream_t st, const RunCfg &cfg, int 
     }
     if (dmc && mv.e == 0) {
       {
-        ProfScope ps(h, QMCB_KERNEL_BRANCH, st);
+        ProfScope ps(h, QMCB_KERNEL_BRANCH, st, prof);
         k_branch<<<1, 1024, 0, st>>>(h->d_state, h->lay, h->d_live, h->d_live_tmp, h->d_free, h->d_ctl,
                                      h->d_copies, h->params.branching_threshold, h->params.fusion_threshold,
                                      h->params.seed, step, h->d_stats, cfg.e_orig, cfg.limit_branching);
         ps.end(st);
       }
       {
-        ProfScope ps(h, QMCB_KERNEL_COPY, st);
+        ProfScope ps(h, QMCB_KERNEL_COPY, st, prof);
         k_copy<<<592, 256, 0, st>>>(h->d_state, h->lay, h->d_copies, h->d_ctl);
         ps.end(st);
       }
       {
-        ProfScope ps(h, QMCB_KERNEL_ENERGY, st);
+        ProfScope ps(h, QMCB_KERNEL_ENERGY, st, prof);
         k_energy<<<1, 32, 0, st>>>(h->d_ectl, h->d_stats, 1, cfg.dyn_dt, cfg.dt);
         ps.end(st);
       }
     }
     if (h->params.refresh_interval > 0 && (step + 1) % h->params.refresh_interval == 0) {
       EvalOut o2{};
-      ProfScope ps(h, QMCB_KERNEL_REFRESH, st);
+      ProfScope ps(h, QMCB_KERNEL_REFRESH, st, prof);
       if (h->md)
         CK(launch_full_md(h, blocks_full, st, cfg, h->d_live, 0, h->d_ctl, nullptr, 0, o2));
       else
@@ -2072,7 +2074,7 @@ static int enqueue_steps(qmcb_handle *h, int first_step, int n_steps, double *du
   RunCfg cfg = make_cfg(h->params);
   // per-call sums; the running E_est sums persist across calls
   CK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_RUN_SUM_W, st));
-  const int rc = launch_steps(h, st, cfg, first_step, n_steps, dump);
+  const int rc = launch_steps(h, st, cfg, first_step, n_steps, dump, true);
   if (rc) return rc;
   const int slot = (h->head + h->n_flight) & 1;
   CK(cudaMemcpyAsync(h->h_stats + slot * ST_COUNT, h->d_stats, sizeof(double) * ST_COUNT, cudaMemcpyDeviceToHost, st));
@@ -2341,6 +2343,7 @@ struct qmcb_group {
   std::vector<std::vector<Bucket>> cands;  // launch configurations the tuner tries
   std::vector<double> cost;                // ms per walker-move of each (< 0: not yet timed)
   int chosen = -1;                         // the tuned configuration
+  bool untimed = false;                    // chosen without timing: no member used its buckets
   int last = -1;                           // configuration of the last batch
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t fork_ev = nullptr;
@@ -2747,7 +2750,15 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
   if (g->cbase >= 0)
     GK(group_upload_const(g->h_gm.data(), nm, g->cbase, st));
   for (auto *h : g->mem) GK(cudaMemsetAsync(h->d_stats, 0, sizeof(double) * ST_RUN_SUM_W, st));
-  // configuration: the tuned one, else the next one not yet timed
+  // configuration: the tuned one, else the next one not yet timed (any while
+  // no member is in a bucket)
+  if (!others && g->chosen < 0) {
+    g->chosen = 0;
+    g->untimed = true;
+  } else if (others && g->untimed) {
+    g->chosen = g->cands.size() == 1 ? 0 : -1;
+    g->untimed = false;
+  }
   int c = g->chosen;
   if (c < 0)
     for (size_t k = 0; k < g->cost.size(); k++)
@@ -2760,7 +2771,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     if (!g->sweeps[i]) continue;
     qmcb_handle *h = g->mem[i];
     GK(cudaStreamWaitEvent(h->stream, g->ev0, 0));
-    const int rc = launch_steps(h, h->stream, make_cfg(h->params), first_steps[g->user[i]], n_steps, nullptr);
+    const int rc = launch_steps(h, h->stream, make_cfg(h->params), first_steps[g->user[i]], n_steps, nullptr, false);
     if (rc) return gfail(g, rc, "qmcb_group_run_steps: member " + std::to_string(g->user[i]) + ": " + h->err);
     if (!g->sweep_ev[i]) GK(cudaEventCreateWithFlags(&g->sweep_ev[i], cudaEventDisableTiming));
     GK(cudaEventRecord(g->sweep_ev[i], h->stream));
@@ -2800,9 +2811,9 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     int rc = group_enqueue(g, c, n_steps, first_steps, refresh);
     if (rc) return rc;
   }
+  GK(cudaEventRecord(g->ev1, st));  // the buckets' end: the configurations differ in nothing else
   for (int i = 0; i < nm; i++)
     if (g->sweeps[i]) GK(cudaStreamWaitEvent(st, g->sweep_ev[i], 0));
-  GK(cudaEventRecord(g->ev1, st));
   for (auto *h : g->mem) {
     GK(cudaMemcpyAsync(h->h_stats, h->d_stats, sizeof(double) * ST_COUNT, cudaMemcpyDeviceToHost, st));
     GK(cudaMemcpyAsync(h->h_ctl, h->d_ctl, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
@@ -2818,7 +2829,7 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     qmcb_handle *h = g->mem[i];
     const double *sv = h->h_stats;
     h->n_live_host = h->h_ctl[0];
-    moves += sv[ST_MOVES];
+    if (!g->sweeps[i]) moves += sv[ST_MOVES];
     if (stats) {
       qmcb_step_stats &s = stats[g->user[i]];
       s.sum_weight = sv[ST_SUM_W];
@@ -2858,6 +2869,7 @@ int qmcb_group_set_config(qmcb_group *g, int config)
 {
   if (!g) return QMCB_E_ARG;
   if (config < -1 || config >= (int)g->cands.size()) return gfail(g, QMCB_E_ARG, "qmcb_group_set_config: no such configuration");
+  g->untimed = false;
   if (config == -1) {
     g->cost.assign(g->cands.size(), -1.0);
     g->chosen = -1;

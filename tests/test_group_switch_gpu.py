@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from qmcbeaver_b200.api import QMCB200Group
-from qmcbeaver_b200.desc import QMCB_DMC, run_params
+from qmcbeaver_b200.desc import QMCB_DMC
 from qmcbeaver_b200.system import make_random_molecule, with_three_body
 from test_group_gpu import _dmc_params, _handles, _params
 
@@ -44,4 +44,22 @@ def test_vmc_then_dmc_without_refreshes():
         a, b = f.get_walkers(), h.get_walkers()
         assert np.array_equal(a["R"], b["R"])
         assert np.allclose(a["weight"], b["weight"], rtol=1e-9)
+    g.close()
+
+
+def test_sweeping_members_alone_need_no_tuning():
+    """Members of small spins run on streams of their own, whatever the launch
+    configuration of the others: nothing to try, and nothing of theirs enters
+    the kernel statistics of their own calls."""
+    systems = [x for k, x in enumerate(_systems()) if k == 0] * 2
+    grouped = _handles(systems, _params)
+    for f in grouped:
+        f.set_profiling(True)
+    g = QMCB200Group(grouped)
+    g.run_steps(0, 12)
+    assert g.config()["chosen"] >= 0
+    for f in grouped:
+        assert all(v["launches"] == 0 for v in f.kernel_stats().values())
+        f.run_steps(12, 3)
+        assert f.kernel_stats()["move"]["launches"] == 1
     g.close()
