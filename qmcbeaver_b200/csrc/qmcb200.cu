@@ -2332,6 +2332,7 @@ struct qmcb_group {
   cudaStream_t stream = nullptr;
   std::vector<qmcb_handle *> mem;  // in launch order (extras flag, then per-warp scratch)
   std::vector<int> user;           // mem[i] is the caller's member user[i]
+  std::vector<char> extras;        // mem[i] was ordered as one of the extras kernels
   GroupMember *d_gm = nullptr;
   std::vector<GroupMember> h_gm;
   int *d_counter = nullptr;  // one per bucket
@@ -2441,6 +2442,28 @@ static int bucket_grid(qmcb_group *g, bool extras, bool ginv, bool md, int strid
   if (per_sm < 1) return gfail(g, QMCB_E_LIMIT, "qmcb_group: a member's scratch does not fit one block");
   *grid = per_sm * g->n_sm;
   return QMCB_OK;
+}
+
+// Members in launch order; noted with it: which take the extras kernels.
+static void order_members(qmcb_group *g)
+{
+  const auto mem = g->mem;
+  const auto user = g->user;
+  std::vector<int> idx(mem.size());
+  for (size_t i = 0; i < idx.size(); i++) idx[i] = (int)i;
+  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
+    if (mem[a]->md != mem[b]->md) return !mem[a]->md;
+    const bool ea = member_extras(mem[a]), eb = member_extras(mem[b]);
+    if (ea != eb) return !ea;
+    if (mem[a]->ginv != mem[b]->ginv) return !mem[a]->ginv;
+    return member_stride(mem[a]) < member_stride(mem[b]);
+  });
+  g->extras.assign(mem.size(), 0);
+  for (size_t i = 0; i < idx.size(); i++) {
+    g->mem[i] = mem[idx[i]];
+    g->user[i] = user[idx[i]];
+    g->extras[i] = member_extras(g->mem[i]);
+  }
 }
 
 // The configurations the tuner tries: members in runs of equal extras flag,
@@ -2605,19 +2628,11 @@ int qmcb_group_create(qmcb_handle *const *members, int n, qmcb_group **out)
   cudaSetDevice(g->device);
   cudaDeviceGetAttribute(&g->n_sm, cudaDevAttrMultiProcessorCount, g->device);
   cudaDeviceGetAttribute(&g->max_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, g->device);
-  std::vector<int> idx(n);
-  for (int i = 0; i < n; i++) idx[i] = i;
-  std::stable_sort(idx.begin(), idx.end(), [&](int a, int b) {
-    if (members[a]->md != members[b]->md) return !members[a]->md;
-    const bool ea = member_extras(members[a]), eb = member_extras(members[b]);
-    if (ea != eb) return !ea;
-    if (members[a]->ginv != members[b]->ginv) return !members[a]->ginv;
-    return member_stride(members[a]) < member_stride(members[b]);
-  });
-  for (int i : idx) {
+  for (int i = 0; i < n; i++) {
     g->mem.push_back(members[i]);
     g->user.push_back(i);
   }
+  order_members(g);
   int rc = QMCB_OK;
   cudaError_t e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaMalloc(&g->d_gm, sizeof(GroupMember) * n);
@@ -2710,6 +2725,19 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     rows_members |= batched_rows(h);
   }
   cudaSetDevice(g->device);
+  // a member's sampling may have changed which kernel it needs: new buckets
+  bool reorder = false;
+  for (int i = 0; i < nm; i++) reorder |= (bool)g->extras[i] != member_extras(g->mem[i]);
+  if (reorder) {
+    if (g->gexec) {
+      cudaGraphExecDestroy(g->gexec);
+      g->gexec = nullptr;
+    }
+    order_members(g);
+    const int rc = build_candidates(g);
+    if (rc) return rc;
+    for (int i = 0; i < nm; i++) g->sweeps[i] = sweep_steps(g->mem[i]);
+  }
   // members' tables, parameters and step numbers
   g->h_gm.assign(nm, GroupMember{});
   for (int i = 0; i < nm; i++) {
@@ -2736,13 +2764,15 @@ int qmcb_group_run_steps(qmcb_group *g, const int *first_steps, int n_steps, qmc
     G.thr_fuse = h->params.fusion_threshold;
   }
   cudaStream_t st = g->stream;
-  if (rows_members && g->rows_ev.empty()) {
+  if (rows_members) {
     size_t nb = 0;
     for (const auto &cand : g->cands) nb = std::max(nb, cand.size());
-    g->step_ev.assign(nb, nullptr);
-    g->rows_ev.assign(nm, nullptr);
-    for (auto &e : g->step_ev) GK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    for (auto &e : g->rows_ev) GK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (auto [evs, n] : {std::pair{&g->step_ev, nb}, std::pair{&g->rows_ev, (size_t)nm}})
+      while (evs->size() < n) {
+        cudaEvent_t e = nullptr;
+        GK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        evs->push_back(e);
+      }
   }
   // the members' own streams finish first (their last evaluate or copy)
   for (auto *h : g->mem) GK(cudaStreamSynchronize(h->stream));

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 
 from qmcbeaver_b200.api import QMCB200Group
-from qmcbeaver_b200.desc import QMCB_DMC
+from qmcbeaver_b200.desc import QMCB_DMC, QMCB_IMPORTANCE_SAMPLING, QMCB_UMRIGAR93_IMPORTANCE_SAMPLING
 from qmcbeaver_b200.system import make_random_molecule, with_three_body
 from test_group_gpu import _dmc_params, _handles, _params
 
@@ -62,4 +62,23 @@ def test_sweeping_members_alone_need_no_tuning():
         assert all(v["launches"] == 0 for v in f.kernel_stats().values())
         f.run_steps(12, 3)
         assert f.kernel_stats()["move"]["launches"] == 1
+    g.close()
+
+
+def test_sampling_switched_after_the_group_was_made():
+    systems = _systems()
+    solo, grouped = _handles(systems, _params), _handles(systems, _params)
+    g = QMCB200Group(grouped)
+    step = 0
+    for sampling in (QMCB_IMPORTANCE_SAMPLING, QMCB_UMRIGAR93_IMPORTANCE_SAMPLING, QMCB_IMPORTANCE_SAMPLING):
+        for k, (f, h) in enumerate(zip(solo, grouped)):
+            f.set_params(_params(k, sampling))
+            h.set_params(_params(k, sampling))
+        for _ in range(3):
+            g.run_steps(step, 11)
+            for f in solo:
+                f.run_steps(step, 11)
+            step += 11
+        for f, h in zip(solo, grouped):
+            assert np.array_equal(f.get_walkers()["R"], h.get_walkers()["R"]), sampling
     g.close()
