@@ -618,7 +618,22 @@ static bool rows_mode(int prec)
 // Whether FP64 moves of `cap` list entries take their rows from k_rows64.
 static bool rows64_moves(const qmcb_handle *h, int cap)
 {
-  return h->params.precision == QMCB_PREC_FP64 && cap >= h->rows64_from;
+  return h->params.precision == QMCB_PREC_FP64 && h->d_rows64 && cap >= h->rows64_from;
+}
+
+// The buffer of k_rows64's rows: with the handle where its FP64 moves may take
+// them, and for a handle whose moves the sweep kernel runs once it gets
+// Umrigar93 moves.  A handle that just fits has none, and moves by the fused
+// kernel.
+static cudaError_t rows64_buffer(qmcb_handle *h)
+{
+  if (h->d_rows64 || h->r64.nchunk == 0) return cudaSuccess;
+  const cudaError_t e = cudaMalloc(&h->d_rows64, sizeof(double) * (size_t)h->max_walkers * 5 * h->nmax);
+  if (e != cudaErrorMemoryAllocation) return e;
+  cudaGetLastError();
+  h->d_rows64 = nullptr;
+  h->rows64_from = INT_MAX;
+  return cudaSuccess;
 }
 
 // Whether k_sweep runs the FP64 moves: at every size (us a step, 1 / 512 /
@@ -1514,16 +1529,7 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
     CKC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, move_fn(true, false, h->extras, h->ginv),
                                                       32 * h->wpb_move, h->smem_move));
     h->rows64_from = h->nmax > 64 ? 1 : n_sm * per_sm * h->wpb_move + 1;
-    if (max_walkers >= h->rows64_from) {
-      const cudaError_t e = cudaMalloc(&h->d_rows64, sizeof(double) * (size_t)max_walkers * 5 * h->nmax);
-      if (e == cudaErrorMemoryAllocation) {
-        cudaGetLastError();  // walkers that just fit: moves by the fused kernel
-        h->d_rows64 = nullptr;
-        h->rows64_from = INT_MAX;
-      } else {
-        CKC(e);
-      }
-    }
+    if (!h->sweep) CKC(rows64_buffer(h));
   }
   // the memsets above ran on the legacy default stream, which does not order
   // against the handle's non-blocking stream: finish them before any work is
@@ -1582,6 +1588,9 @@ int qmcb_set_params(qmcb_handle *h, const qmcb_run_params *p)
     const int rc = rows_bf_setup(h);
     if (rc) return rc;
   }
+  if (p->precision == QMCB_PREC_FP64 && p->sampling == QMCB_UMRIGAR93_IMPORTANCE_SAMPLING &&
+      h->max_walkers >= h->rows64_from)
+    CK(rows64_buffer(h));
   h->params = *p;
   if (h->n_live_host > 0) {
     // the host's E_T / E_est feed the next steps (QMCManager::updateTrialEnergy)
@@ -2165,6 +2174,7 @@ size_t qmcb_state_bytes(const qmcb_handle *h)
 {
   if (!h) return 0;
   size_t b = (size_t)h->max_walkers * h->lay.stride * sizeof(double);
+  if (h->d_rows64) b += sizeof(double) * (size_t)h->max_walkers * 5 * h->nmax;
   // the tensor-core rows modes' buffers, once a mode has set them up
   const size_t tiles = (size_t)(h->max_walkers + kTileWalkers - 1) / kTileWalkers;
   if (h->d_rows_out) b += sizeof(double) * (size_t)h->max_walkers * 5 * h->nmax;

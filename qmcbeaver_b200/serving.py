@@ -76,8 +76,9 @@ def state_footprint(system: MolecularSystem, walkers: int, precision: int = QMCB
     (the per-walker block of the library, 2x walker capacity, 256-byte
     blocks): positions, Slater rows / derivatives / inverse per spin (two
     inverse copies for spins above 16 electrons), per-electron arrays,
-    scalars; for the tensor-core rows modes also their operand planes, block
-    scales and the step's rows (the library's qmcb_state_bytes)."""
+    scalars; the step's orbital rows where FP64 moves may take them from the
+    batched kernel; for the tensor-core rows modes also their operand planes,
+    block scales and the step's rows (the library's qmcb_state_bytes)."""
     def pad4(x):
         return (x + 3) & ~3
     N, na, nb = system.n_electrons, system.n_alpha, system.n_beta
@@ -89,6 +90,8 @@ def state_footprint(system: MolecularSystem, walkers: int, precision: int = QMCB
     words = (words + 31) & ~31
     cap = 2 * walkers
     total = cap * words * 8
+    if system.n_det == 1 and (max(na, nb) > 16 or system.replace_cusps or system.three_body):
+        total += 8 * cap * 5 * max(na, nb)         # no sweep kernel: the step's FP64 rows
     if precision in (QMCB_PREC_INT8_SLICES, QMCB_PREC_BF16_TC, QMCB_PREC_BF16X3_TC):
         K = system.n_basis
         tiles = -(-cap // 25)                      # 25 walkers (125 of 128 rows) per tile
