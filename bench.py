@@ -736,17 +736,22 @@ def main():
                              st.final_weight)
 
     # roofline of the move kernel (dominant; a launch runs all the steps between
-    # two branchings or refreshes): algorithmic bytes per launch / launch time
+    # two branchings or refreshes, its walkers on the chip): the DRAM bytes that
+    # the committed profile counts per move / launch time.  The kernel is bound
+    # by the latency of a step's chain and its issue, far below HBM; what a step
+    # by itself could not do without (bytes_per_move) is given beside it.
     mv = ks["move"]
     avg_ms = mv["ms"] / max(mv["launches"], 1)
     moves_per_launch = st.n_moves / max(mv["launches"], 1)
     bpm = bytes_per_move(n, N)
-    achieved = bpm * moves_per_launch / (avg_ms / 1e3) / 1e9
+    rate = moves_per_launch / (avg_ms / 1e3)
     peak, peak_kind = read_peaks()
     tr = read_traffic(WORKLOAD)
-    roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+    achieved = (tr if tr is not None else bpm) * rate / 1e9
+    roofline = {"bound": "latency", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": (tr * moves_per_launch) if tr is not None else None,
                 "peak_kind": peak_kind, "kernel": "k_sweep", "algorithmic_bytes_per_walker_move": bpm,
+                "algorithmic_gbs_step_by_step": bpm * rate / 1e9,
                 "moves_per_launch": moves_per_launch, "avg_launch_ms": avg_ms}
     launches = int(sum(v["launches"] for v in ks.values()))
 

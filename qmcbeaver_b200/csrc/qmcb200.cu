@@ -72,7 +72,7 @@ struct qmcb_handle {
   int bf_ksteps = 0;
   int rows_n = 0, rows_num = 0;  // the last tensor-core rows launch: orbitals per row, list capacity
   size_t smem_rows = 0, smem_prep = 0;
-  // batched FP64 rows (kernels_rows64.cuh): tables, rows buffer [walker][5][n]
+  // batched FP64 rows (rows64.cu): tables, rows buffer [walker][5][n]
   Rows64 r64{};
   int rows64_from = INT_MAX;  // FP64 single-electron moves of this many walkers take their rows from k_rows64
   int4 *d_r64_chunk = nullptr;
@@ -1383,8 +1383,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   for (int sp = 0; sp < 2; sp++) {
     int n = sp ? nb : na, a = nact[sp];
     L.Dv[sp] = take(n * a);
-    L.D4[sp] = take(3 * a * n);  // (the block's size predates the interleaved elements: 3 + 1 per pair, padded apart)
-    take(a * n);
+    L.D4[sp] = take(3 * a * n);  // [a][n][4]: 3 + 1 doubles a pair, rounded up apart,
+    take(a * n);                 // as the block size that callers count with has it
     if (md) {
       // two copies of [inverses | grad ratios | (ln|det|, sign, lap, singular)]
       L.mdsz[sp] = (S.ndet * n * n + S.ndet * 3 * n + S.ndet * 4 + 3) & ~3;
@@ -2333,7 +2333,7 @@ int qmcb_branch_weights_noalloc(const double *d_weight_in, int n, double branchi
 // ------------------------------------------------------------------------
 // Groups: the walkers of many handles (systems of different sizes) stepped
 // by one persistent launch per bucket of similar shared-memory need
-// (kernels_group.cuh).  No counterpart in the reference, which runs one
+// (group.cu).  No counterpart in the reference, which runs one
 // molecule per process.
 
 struct qmcb_group {
