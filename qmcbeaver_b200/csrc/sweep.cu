@@ -28,7 +28,7 @@
 // (The laplacian's sum over the columns and the acceptance's exponents, which
 // feed nothing back, add in the lanes' own order, and so does the one sum of
 // the drift limited by a common factor, qf_mod 1.)  150 steps of 16,384 walkers
-// of 30 electrons take 16.7 ms so, 16.0 with sums in the cheapest order.
+// of 30 electrons take 16.1 ms so, 15.9 with sums in the cheapest order.
 //
 // Bound by the latency of a step's chain of phases (30 electrons: 40 k cycles
 // with one CTA per SM -- proposals 1, basis 7.5, products 6, pair terms 3,
@@ -39,7 +39,7 @@
 // registers a thread; with 223 KB of shared memory the L1 is small, so spilled
 // registers cost L2 latencies and the column of the inverse leaves the
 // registers for the ratio sums.  30 electrons, 15,710 walkers: 225 us a step
-// by the move kernel, 90 here; 10 electrons, 100 walkers: 18 and 9.
+// by the move kernel, 87 here; 10 electrons, 100 walkers: 18 and 9.
 #include "rows64_device.cuh"
 #include "sweep.h"
 
@@ -148,6 +148,39 @@ __device__ __forceinline__ void pair_change(const DevSys &S, int f, double k, bo
   for (int d = 0; d < 3; d++) v[d] = sn * xn[d] - so * xo[d];
 }
 
+// The moved electron's change with nucleus A (none from M on), added to the
+// sums w: dU, lap, V_ee, V_en, gradient on it.
+__device__ __forceinline__ void nuclear_changes(const DevSys &S, int sp, int A, int M, const double ro[3],
+                                                const double rn[3], double w[7])
+{
+  const double4 P = S.nuc[A < M ? A : 0];
+  const double p[3] = {P.x, P.y, P.z};
+  double v[3], dinv;
+  pair_change(S, S.en[sp][A < M ? A : 0], 1.0, A < M, ro, rn, p, dinv, w[0], w[1], v);
+  w[3] -= P.w * dinv;
+#pragma unroll
+  for (int d = 0; d < 3; d++) w[4 + d] += v[d];
+}
+
+// The nuclei of more than a walker's lanes hold: those of the move kernel's
+// lanes c and G + c (w[0..7), w[7..14), which hold their electrons' sums) and of
+// the two lanes 2 G + c, 3 G + c of a group of eight, nuclei l, l + 32, .. each;
+// then the sums over these in the order of warp_sum, in w[0..7).
+template <int G>
+static __device__ __noinline__ void many_nuclei(const DevSys &S, int sp, int c, const double ro[3], const double rn[3],
+                                                double w[14])
+{
+  for (int half = 0; half < 2; half++)
+    for (int A = G * half + c; A - c < S.M; A += 32) nuclear_changes(S, sp, A, S.M, ro, rn, w + 7 * half);
+  if (G == 8)
+    for (int half = 0; half < 2; half++) {
+      double x[7] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+      for (int A = 2 * G + G * half + c; A - c < S.M; A += 32) nuclear_changes(S, sp, A, S.M, ro, rn, x);
+      for (int k = 0; k < 7; k++) w[7 * half + k] += x[k];
+    }
+  for (int k = 0; k < 7; k++) w[k] += w[7 + k];
+}
+
 // Shared memory of a CTA (offsets in doubles): the chunk of basis values (the
 // moved spin's inverses once it is consumed), two coefficient buffers,
 // positions [3][TW], displacements [3][TW], acceptance uniforms [TW], rows
@@ -231,49 +264,36 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
       ro[d] = sR[3 * e + d];
       rn[d] = sm[Sh::kPos + TW * d + gi];
     }
-    // the lanes l = c, G + c (and from 2 G on, for more nuclei than that) of
-    // jastrow_pe_move_warp: electron l, then nuclei l, l + 32, ..
-    double u[7];
-    const auto electron = [&](int s, double w[7]) {
+    // the lanes c and G + c of jastrow_pe_move_warp one after another: lane l's
+    // electron l, then nucleus l
+    double u[3];
+    const auto electron = [&](int s, double &dU, double &dUxx, double &dVee) {
       const double *r = sR + (has[s] ? 3 * idx[s] : 0), P[3] = {r[0], r[1], r[2]};
-      w[0] = w[1] = 0.0;
+      dU = dUxx = 0.0;
       pair_change(S, (idx[s] < S.na ? 0 : 1) != sp ? S.ee[0] : sp == 0 ? S.ee[1] : S.ee[2], 2.0,
-                  has[s] && idx[s] != e, ro, rn, P, w[2], w[0], w[1], vx[s]);
-      w[3] = 0.0;
-#pragma unroll
-      for (int d = 0; d < 3; d++) w[4 + d] = vx[s][d];
+                  has[s] && idx[s] != e, ro, rn, P, dVee, dU, dUxx, vx[s]);
     };
-    const auto nuclei = [&](int l0, double w[7]) {
-      for (int A0 = l0; A0 < S.M; A0 += 32) {
-        const int A = A0 + c < S.M ? A0 + c : 0;
-        const double4 P = S.nuc[A];
-        const double p[3] = {P.x, P.y, P.z};
-        double v[3], dinv;
-        pair_change(S, S.en[sp][A], 1.0, A0 + c < S.M, ro, rn, p, dinv, w[0], w[1], v);
-        w[3] -= P.w * dinv;
+    electron(0, s8[0], s8[1], s8[2]);
+    electron(1, u[0], u[1], u[2]);
+    s8[3] = 0.0;
 #pragma unroll
-        for (int d = 0; d < 3; d++) w[4 + d] += v[d];
-      }
-    };
-    electron(0, s8);
-    electron(1, u);
-    nuclei(0, s8);
-    if (S.M > G) nuclei(G, u);
-    if (G == 8 && S.M > 2 * G) {
-      double w[7];
+    for (int d = 0; d < 3; d++) s8[4 + d] = vx[0][d];
+    if (S.M <= G) {
+      nuclear_changes(S, sp, c, S.M, ro, rn, s8);
 #pragma unroll
-      for (int k = 0; k < 7; k++) w[k] = 0.0;
-      nuclei(2 * G, w);
+      for (int k = 0; k < 3; k++) s8[k] += u[k];
 #pragma unroll
-      for (int k = 0; k < 7; k++) s8[k] += w[k];
+      for (int d = 0; d < 3; d++) s8[4 + d] += vx[1][d];
+    } else {
+      double w[14];
 #pragma unroll
-      for (int k = 0; k < 7; k++) w[k] = 0.0;
-      nuclei(3 * G, w);
+      for (int k = 0; k < 7; k++) w[k] = s8[k];
 #pragma unroll
-      for (int k = 0; k < 7; k++) u[k] += w[k];
+      for (int k = 0; k < 7; k++) w[7 + k] = k < 3 ? u[k] : k == 3 ? 0.0 : vx[1][k - 4];
+      many_nuclei<G>(S, sp, c, ro, rn, w);
+#pragma unroll
+      for (int k = 0; k < 7; k++) s8[k] = w[k];
     }
-#pragma unroll
-    for (int k = 0; k < 7; k++) s8[k] += u[k];
     s8[7] = gf;
   }
   const double sums1 = group_sum8<G>(s8, c, gm);
@@ -318,11 +338,13 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
     constexpr int kB = 8;
     // slice by slice for the larger spins (2 or 3 of up to 8 orbitals), the
     // whole column in one batch for the smaller (4 or more of up to 2)
-    const int slices = G == 16 ? 32 / n : 1;
+    const int slices = G == 16 ? __popc(slice_ends) : 1;
+    unsigned rest = slice_ends;
+    int oa = 0;
 #pragma unroll 1
     for (int s = 0; s < slices; s++) {
-      const int oa = G == 16 ? n * s / slices : 0, ob = G == 16 ? n * (s + 1) / slices : n;
-      if (oa == ob) continue;
+      const int ob = G == 16 ? __ffs(rest) : n;
+      rest &= rest - 1;
       Deriv4<double> g[kB], part = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
       for (int u = 0; u < kB; u++) g[u] = ld_deriv<false>(D4 + min(oa + u, ob - 1) * n);
@@ -343,6 +365,7 @@ __device__ __forceinline__ void sweep_move(const DevSys &S, const Layout &L, con
           part = {0.0, 0.0, 0.0, 0.0};
         }
       }
+      oa = ob;
     }
     lp = mine ? lp : 0.0;
   }
