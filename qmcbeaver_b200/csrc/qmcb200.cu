@@ -502,6 +502,21 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
     if (doubles(it) >= kR64RecMax) return cudaSuccess;
   const auto first = [](const Item &it) { return *std::min_element(it.members.begin(), it.members.end()); };
   std::sort(items.begin(), items.end(), [&](const Item &a, const Item &b) { return first(a) < first(b); });
+  // a chunk's records leave room for the sweep kernel's CTAs on an SM, two or, of
+  // spins up to 8, four, unless that means chunks of fewer than 16 s shells
+  // (8,192 walkers on s functions alone: 30 electrons 53 us a step, 71 with one CTA;
+  // 14 electrons 20, 30 with three)
+  int longest = kR64RecMax;
+  if (h->nmax <= 16) {
+    int smem_sm = 0, reserved = 0;
+    cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, h->device);
+    cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, h->device);
+    Rows64 none{};
+    none.nchunk = 2 * (h->K / cap + 1);
+    const int room = (smem_sm / (h->nmax > 8 ? 2 : 4) - reserved - 128 - sweep_smem_bytes(h->nmax, h->lay, none)) /
+                     (2 * (int)sizeof(double));
+    if (room >= 160) longest = std::min(longest, room & ~1);
+  }
   std::vector<std::vector<Item>> chunks;
   std::vector<int> fill, size;
   // a shell that does not fit starts the next chunk or (cut) is parted: one of
@@ -518,7 +533,7 @@ static cudaError_t rows64_tables(qmcb_handle *h, const std::vector<int4> &shells
     for (const Item &it : items) {
       const int nmem = (int)it.members.size();
       for (int done = 0; done < nmem;) {
-        const bool full = chunks.empty() || fill.back() == cap || size.back() + doubles(it) >= kR64RecMax;
+        const bool full = chunks.empty() || fill.back() == cap || size.back() + doubles(it) >= longest;
         if (full || (!cut && fill.back() + nmem > cap)) open();
         const int part = std::min(nmem - done, cap - fill.back());
         Item piece = it;
@@ -1271,7 +1286,6 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
   CKC(upload(&h->d_shell, shells));
   CKC(upload(&h->d_fn, fn));
   CKC(upload(&h->d_xsl, xsl));
-  if (!md) CKC(rows64_tables(h, shells, fn, nuc, pexp, pcoef, ct, nact));
   CKC(upload(&h->d_fq, fq));
   CKC(upload(&h->d_pexp, pexp));
   CKC(upload(&h->d_pcoef, pcoef));
@@ -1429,6 +1443,8 @@ int qmcb_create(const qmcb_system_desc *d, int max_walkers, qmcb_handle **out)
     qmcb_destroy(h);
     return fail(nullptr, QMCB_E_ARG, "qmcb_create: internal layout error (staged ranges exceed the walker block)");
   }
+
+  if (!md) CKC(rows64_tables(h, shells, fn, nuc, pexp, pcoef, ct, nact));
 
   size_t bytes = (size_t)max_walkers * L.stride * sizeof(double);
   CKC(cudaMalloc(&h->d_state, bytes));
